@@ -1432,6 +1432,7 @@ static long div_correct(Context &c, int k, bool fp32, const double *b, double *x
     a.y = w.div_me.p;
     a.relax_w = 1.0;
     a.mode = SPMM_AX;
+    a.chained = true;
     spmm_nnz<double>(K2, a, c.nnz, s);
     ams_restrict<double>(nv, K2, 0, c.vinc_rp.p, c.vinc.p, nullptr, w.div_me.p, w.div_u.p, s);
     vrow_scale<double, double>(nv, K2, w.div_dis.p, w.div_u.p, s_, s);
@@ -1534,6 +1535,7 @@ static void solve_block_pow2(Context &c, int k, const double *freqs, const doubl
     a.y = s_;
     a.relax_w = 1.0;
     a.mode = SPMM_AX;
+    a.chained = true;
     KernelProfiler &pf = profiler();
     cudaEvent_t ev = nullptr, ph = nullptr;
     if (pf.enabled)

@@ -29,7 +29,7 @@ void spmm_launch(const SpmmArgs &a, cudaStream_t s) {
   long threads = warps * 32;
   unsigned grid = (unsigned)((threads + 255) / 256);
   if (grid == 0) return;
-  spmm_kernel<T, K, V, NL, PK, MINB><<<grid, 256, 0, s>>>(a);
+  launch_chain(&spmm_kernel<T, K, V, NL, PK, MINB>, grid, 256, s, a.chained, a);
 }
 
 // register-capped row-split kernel (nl = 400 + NL packed records, 500 + NL
@@ -55,7 +55,7 @@ void spmm_rows_launch(const SpmmArgs &a, cudaStream_t s) {
   long warps = ((long)a.n + RPW - 1) / RPW;
   unsigned grid = (unsigned)((warps * 32 + 255) / 256);
   if (grid == 0) return;
-  spmm_rows_kernel<T, K, V, B><<<grid, 256, 0, s>>>(a);
+  launch_chain(&spmm_rows_kernel<T, K, V, B>, grid, 256, s, a.chained, a);
 }
 
 template <typename T, int K, int V, int B>
@@ -72,7 +72,7 @@ void spmm_pipe_launch(const SpmmArgs &a, cudaStream_t s) {
   long warps = ((long)a.n + RPW - 1) / RPW;
   unsigned grid = (unsigned)((warps * 32 + 255) / 256);
   if (grid == 0) return;
-  spmm_pipe_kernel<T, K, V, U, PK><<<grid, 256, 0, s>>>(a);
+  launch_chain(&spmm_pipe_kernel<T, K, V, U, PK>, grid, 256, s, a.chained, a);
 }
 
 template <typename T, int K, int V, int U, bool PK>
@@ -90,7 +90,7 @@ void spmm_chunk_launch(const SpmmArgs &a, cudaStream_t s) {
   long warps = ((long)a.n + RPW - 1) / RPW;
   unsigned grid = (unsigned)((warps * 32 + 255) / 256);
   if (grid == 0) return;
-  spmm_chunk_kernel<K, V, MINB><<<grid, 256, 0, s>>>(a);
+  launch_chain(&spmm_chunk_kernel<K, V, MINB>, grid, 256, s, a.chained, a);
 }
 
 template <typename T, int K, int V, int MINB>
@@ -193,6 +193,14 @@ static int row_bucket(const SpmmArgs &a, long nnz) {
 // row-count class: the edge matrix and the finest nodal levels tune apart
 static int size_class(const SpmmArgs &a) { return a.n >= 1000000 ? 2 : (a.n >= 100000 ? 1 : 0); }
 
+// Layout of an operator whose rows x column lanes leave most of the chip idle
+// (a quarter of its threads): the widest vectors, and as many lanes per row
+// as bring it down to one round of 4 nonzeros per lane, because there a step
+// costs its dependent loads and not its bandwidth.  An operator of 240 rows
+// with 30 nonzeros (K = 32) takes 6.5 us this way and 15.7 us with one lane
+// per row, the layout that wins at 20000 rows.
+constexpr long kLaneSlots = 148L * 512;
+
 template <typename T>
 static std::pair<int, int> spmm_default(int K, double avg) {
   int vmax = (int)(16 / sizeof(T));
@@ -201,7 +209,7 @@ static std::pair<int, int> spmm_default(int K, double avg) {
   int cl = K / v;
   while (cl > 32) { v *= 2; cl = K / v; }
   int nl = 1;
-  while (nl * 2 * cl <= 32 && nl * 2 <= std::max(1.0, avg / 2)) nl *= 2;
+  while (nl * 2 * cl <= 32 && nl * 4 < avg) nl *= 2;
   return {v, nl};
 }
 
@@ -215,15 +223,16 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
   auto key = std::make_tuple((int)sizeof(T), K, bucket, 4 * size_class(a) + (packed ? 1 : 0) + (chunked ? 2 : 0));
   auto it = tn.best.find(key);
   std::pair<int, int> cfg;
-  if (it != tn.best.end()) {
+  if (it != tn.best.end() && (long)a.n * (K / spmm_default<T>(K, 1.0).first) >= kLaneSlots) {
     cfg = it->second;
   } else {
     cfg = spmm_default<T>(K, a.n ? (double)nnz / a.n : 1.0);
+    const bool fills = (long)a.n * (K / cfg.first) >= kLaneSlots;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     EMG_CUDA(cudaStreamIsCapturing(s, &cs));
     const bool idempotent = a.mode == SPMM_AX || a.mode == SPMM_RES || a.mode == SPMM_JAC || a.mode == SPMM_CHEB1 ||
-                            a.mode == SPMM_AXJ0;
-    if (tn.allow_tuning && cs == cudaStreamCaptureStatusNone && idempotent && a.n >= 20000) {
+                            a.mode == SPMM_AXJ0 || a.mode == SPMM_RESJ0;
+    if (tn.allow_tuning && cs == cudaStreamCaptureStatusNone && idempotent && fills) {
       cudaEvent_t e0, e1;
       EMG_CUDA(cudaEventCreate(&e0));
       EMG_CUDA(cudaEventCreate(&e1));
@@ -244,9 +253,11 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
       for (int pass = 0; pass < 2; ++pass)
         for (size_t i = 0; i < cand.size(); ++i) {
           SpmmFn f = spmm_fn<T>(K, cand[i].first, cand[i].second);
-          f(a, s);  // warm-up
+          SpmmArgs ta = a;
+          ta.chained = false;
+          f(ta, s);  // warm-up
           EMG_CUDA(cudaEventRecord(e0, s));
-          for (int r = 0; r < 3; ++r) f(a, s);
+          for (int r = 0; r < 3; ++r) f(ta, s);
           EMG_CUDA(cudaEventRecord(e1, s));
           EMG_CUDA(cudaEventSynchronize(e1));
           float ms = 0;
@@ -396,7 +407,8 @@ double spmm_algo_bytes(long n, long nnz, int K, int elem, bool two_parts, int mo
   if (mode == SPMM_CHEB1) b += 3.0 * vec + (double)n * elem * (two_parts ? 2 : 1);   // b, x-row in; r, d out
   if (mode == SPMM_CHEB2) b += 2.0 * vec + (double)n * elem * (two_parts ? 2 : 1);   // r, y-row in
   if (mode == SPMM_CHEBK) b += 4.0 * vec + (double)n * elem * (two_parts ? 2 : 1);   // r, y in; r, d out
-  if (mode == SPMM_AXJ0) b += 2.0 * vec + (double)n * elem * 2;                      // r, d out; fed diagonal
+  if (mode == SPMM_RESJ0) b += vec;
+  if (mode == SPMM_AXJ0 || mode == SPMM_RESJ0) b += 2.0 * vec + (double)n * elem * 2;                      // r, d out; fed diagonal
   return b;
 }
 
@@ -522,49 +534,49 @@ void fcg_direction(int n, int K, const T *z, int nprev, T *const *Pj, const doub
   EMG_LAUNCH_CHECK();
 }
 
+// columns per vector load of a K-column block row
 template <typename T>
-__global__ void jacobi0_kernel(long total, int K, const T *__restrict__ b, const T *__restrict__ l1c,
-                               const T *__restrict__ l1m, const double *__restrict__ omega, double w,
-                               T *__restrict__ y) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+static int vec_width(int K) {
+  return (K & 3) == 0 && sizeof(T) == 4 ? 4 : ((K & 1) == 0 ? 2 : 1);
+}
+
+// y (and d when given) = w b / (l1c + w_c l1m): one thread per V columns of a
+// row; the diagonals load before the wait (emg_pdl.cuh)
+template <typename T, int V>
+__global__ void __launch_bounds__(256) jacobi0_kernel(long total, int cl, const T *b, const T *__restrict__ l1c,
+                                                      const T *__restrict__ l1m, const double *__restrict__ omega,
+                                                      double w, T *y, T *d) {
+  pdl_trigger();
+  const long i = blockIdx.x * 256L + threadIdx.x;
+  T dg[V];
+  if (i < total) {
+    const long row = i / cl;
+    const int c0 = (int)(i - row * cl) * V;
+    const T dc = __ldg(l1c + row), dm = l1m ? __ldg(l1m + row) : T(0);
+#pragma unroll
+    for (int q = 0; q < V; ++q) dg[q] = l1m ? dc + (T)__ldg(omega + c0 + q) * dm : dc;
+  }
+  pdl_wait();
   if (i >= total) return;
-  long row = i / K;
-  int c = (int)(i % K);
-  T d = l1c[row];
-  if (l1m) d += (T)omega[c] * l1m[row];
-  y[i] = (T)w * b[i] / d;
+  T v[V];
+  ldv<T, V>(b + i * V, v);
+#pragma unroll
+  for (int q = 0; q < V; ++q) v[q] = (T)w * v[q] / dg[q];
+  stv<T, V>(y + i * V, v);
+  if (d) stv<T, V>(d + i * V, v);
 }
 
 template <typename T>
-void jacobi0(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y,
+void jacobi0(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y, T *d,
              cudaStream_t s) {
-  long total = (long)n * K;
-  if (!total) return;
-  jacobi0_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(total, K, b, l1c, l1m, omega, w, y);
-  EMG_LAUNCH_CHECK();
-}
-
-template <typename T>
-__global__ void jacobi0_2_kernel(long total, int K, const T *__restrict__ b, const T *__restrict__ l1c,
-                                 const T *__restrict__ l1m, const double *__restrict__ omega, double w,
-                                 T *__restrict__ y, T *__restrict__ d) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  long row = i / K;
-  int c = (int)(i % K);
-  T dg = l1c[row];
-  if (l1m) dg += (T)omega[c] * l1m[row];
-  T v = (T)w * b[i] / dg;
-  y[i] = v;
-  d[i] = v;
-}
-
-template <typename T>
-void jacobi0_2(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y, T *d,
-               cudaStream_t s) {
-  long total = (long)n * K;
-  if (!total) return;
-  jacobi0_2_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(total, K, b, l1c, l1m, omega, w, y, d);
+  if (n <= 0) return;
+  const int v = vec_width<T>(K), cl = K / v;
+  const long total = (long)n * cl;
+  const unsigned grid = (unsigned)((total + 255) / 256);
+  if (v == 1) launch_chain(&jacobi0_kernel<T, 1>, grid, 256, s, true, total, cl, b, l1c, l1m, omega, w, y, d);
+  else if (v == 2) launch_chain(&jacobi0_kernel<T, 2>, grid, 256, s, true, total, cl, b, l1c, l1m, omega, w, y, d);
+  else if constexpr (sizeof(T) == 4)
+    launch_chain(&jacobi0_kernel<T, 4>, grid, 256, s, true, total, cl, b, l1c, l1m, omega, w, y, d);
   EMG_LAUNCH_CHECK();
 }
 
@@ -673,97 +685,227 @@ void fill_zero(long count, T *a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // AMS transfers
 // ---------------------------------------------------------------------------
+// One vertex per CL x NL lanes: CL lanes own V columns each, NL lanes split the
+// incident edges (about 14 per vertex), U of them per lane and round.  The
+// incidence codes and tangents of the first round load before the wait; what
+// remains of the chain is one round of gathers.  With y, the first smoothing
+// step of the level this right-hand side feeds is taken as well: y = d =
+// c1 b / (l1c + w_c l1m), one pass and one launch less per V-cycle.
 template <typename T>
-__global__ void ams_restrict_kernel(int nv, int K, int sp, const int *__restrict__ inc_rp,
-                                    const int *__restrict__ inc, const T *__restrict__ tangent,
-                                    const T *__restrict__ r_edge, T *__restrict__ r_vert) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)nv * K) return;
-  int v = (int)(i / K), c = (int)(i % K);
-  const int kb = __ldg(inc_rp + v), ke = __ldg(inc_rp + v + 1);
-  if (sp == 4) {  // vector space: rows 3 v + d
-    T a0 = 0, a1 = 0, a2 = 0;
-    for (int k = kb; k < ke; ++k) {
-      int e = __ldg(inc + k) >> 1;
-      T r = T(0.5) * __ldg(r_edge + (long)e * K + c);
-      a0 += __ldg(tangent + 3 * (long)e) * r;
-      a1 += __ldg(tangent + 3 * (long)e + 1) * r;
-      a2 += __ldg(tangent + 3 * (long)e + 2) * r;
+struct RestrictArgs {
+  int nv, K, sp, cl, nl;
+  const int *inc_rp, *inc;
+  const T *tangent, *r_edge;
+  T *r_vert;
+  RestrictJ0<T> j0;
+};
+
+template <typename T, int V, int D>
+__global__ void __launch_bounds__(256) ams_restrict_kernel(RestrictArgs<T> a) {
+  constexpr int U = 4;
+  pdl_trigger();
+  const int K = a.K, g = a.cl * a.nl;
+  const long t = (blockIdx.x * 256L + threadIdx.x) / g;
+  const int sub = (int)(threadIdx.x % g), c0 = (sub % a.cl) * V, sl = sub / a.cl;
+  const bool valid = t < a.nv;
+  const int v = (int)t;
+  int k0 = 0, ke = 0;
+  if (valid) {
+    k0 = __ldg(a.inc_rp + v) + sl;
+    ke = __ldg(a.inc_rp + v + 1);
+  }
+  int e[U];
+  T w[U][D];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * a.nl;
+      const int code = k < ke ? __ldg(a.inc + k) : -1;
+      e[u] = code >> 1;  // -1 past the end
+      if (code >= 0) {
+        if constexpr (D == 3) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) w[u][d] = __ldg(a.tangent + 3 * (long)e[u] + d);
+        } else if (a.sp == 0) {
+          w[u][0] = (code & 1) ? T(1) : T(-1);
+        } else {
+          w[u][0] = T(0.5) * __ldg(a.tangent + 3 * (long)e[u] + (a.sp - 1));
+        }
+      }
     }
-    r_vert[(3 * (long)v) * K + c] = a0;
-    r_vert[(3 * (long)v + 1) * K + c] = a1;
-    r_vert[(3 * (long)v + 2) * K + c] = a2;
-    return;
+  };
+  fetch();
+  pdl_wait();
+  T acc[D][V];
+#pragma unroll
+  for (int d = 0; d < D; ++d)
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[d][i] = T(0);
+  while (k0 < ke) {
+    T r[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e[u] >= 0) ldv<T, V>(a.r_edge + (long)e[u] * K + c0, r[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e[u] >= 0)
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+#pragma unroll
+          for (int d = 0; d < D; ++d) acc[d][i] += w[u][d] * (D == 3 ? T(0.5) * r[u][i] : r[u][i]);
+    k0 += a.nl * U;
+    if (k0 < ke) fetch();
   }
-  T acc = 0;
-  for (int k = kb; k < ke; ++k) {
-    int code = __ldg(inc + k);
-    int e = code >> 1;
-    T w;
-    if (sp == 0) w = (code & 1) ? T(1) : T(-1);
-    else w = T(0.5) * __ldg(tangent + 3 * (long)e + (sp - 1));
-    acc += w * __ldg(r_edge + (long)e * K + c);
+  for (int off = a.cl; off < g; off <<= 1)
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[d][i] += __shfl_xor_sync(0xffffffffu, acc[d][i], off);
+  if (!valid || sl != 0) return;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const long row = (long)D * v + d, o = row * K + c0;
+    stv<T, V>(a.r_vert + o, acc[d]);
+    if (a.j0.y) {
+      const T dc = __ldg(a.j0.l1c + row), dm = a.j0.l1m ? __ldg(a.j0.l1m + row) : T(0);
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        acc[d][i] = (T)a.j0.c1 * acc[d][i] / (a.j0.l1m ? dc + (T)__ldg(a.j0.omega + c0 + i) * dm : dc);
+      stv<T, V>(a.j0.y + o, acc[d]);
+      if (a.j0.d) stv<T, V>(a.j0.d + o, acc[d]);
+    }
   }
-  r_vert[i] = acc;
 }
 
 template <typename T>
 void ams_restrict(int nv, int K, int sp, const int *inc_rp, const int *inc, const T *tangent, const T *r_edge,
-                  T *r_vert, cudaStream_t s) {
-  long total = (long)nv * K;
-  ams_restrict_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(nv, K, sp, inc_rp, inc, tangent, r_edge,
-                                                                         r_vert);
+                  T *r_vert, cudaStream_t s, const RestrictJ0<T> &j0) {
+  if (nv <= 0) return;
+  const int v = vec_width<T>(K), cl = K / v;
+  // 4 lanes x 4 edges cover the usual vertex in one round
+  int nl = 1;
+  while (nl < 4 && cl * nl * 2 <= 32) nl *= 2;
+  if (cl > 32 || (32 % cl) != 0) fail(EMG_ERR_ARG, "unsupported block width K=%d", K);
+  RestrictArgs<T> a{nv, K, sp, cl, nl, inc_rp, inc, tangent, r_edge, r_vert, j0};
+  const unsigned grid = (unsigned)(((long)nv * cl * nl + 255) / 256);
+  auto run = [&](auto k1, auto k3) { launch_chain(sp == 4 ? k3 : k1, grid, 256, s, true, a); };
+  if (v == 1) run(&ams_restrict_kernel<T, 1, 1>, &ams_restrict_kernel<T, 1, 3>);
+  else if (v == 2) run(&ams_restrict_kernel<T, 2, 1>, &ams_restrict_kernel<T, 2, 3>);
+  else if constexpr (sizeof(T) == 4) run(&ams_restrict_kernel<T, 4, 1>, &ams_restrict_kernel<T, 4, 3>);
   EMG_LAUNCH_CHECK();
 }
 
-template <typename T>
-__global__ void ams_prolong_kernel(int ne, int K, int sp, const int *__restrict__ edges,
-                                   const T *__restrict__ tangent, const T *__restrict__ ev, T *__restrict__ x) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)ne * K) return;
-  int e = (int)(i / K), c = (int)(i % K);
-  int v0 = __ldg(edges + 2 * (long)e), v1 = __ldg(edges + 2 * (long)e + 1);
-  T val;
-  if (sp == 4) {  // vector space: rows 3 v + d
-    val = 0;
+// x += Q e: one thread per V columns of an edge; end points and tangent load
+// before the wait
+template <typename T, int V>
+__global__ void __launch_bounds__(256) ams_prolong_kernel(int ne, int K, int cl, int sp, const int *__restrict__ edges,
+                                                          const T *__restrict__ tangent, const T *ev, T *x) {
+  pdl_trigger();
+  const long t = blockIdx.x * 256L + threadIdx.x;
+  const bool valid = t < (long)ne * cl;
+  int2 vv = make_int2(0, 0);
+  T tg[3] = {T(0), T(0), T(0)};
+  long e = 0;
+  if (valid) {
+    e = t / cl;
+    vv = __ldg(reinterpret_cast<const int2 *>(edges) + e);
+    if (sp == 4) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-      val += __ldg(tangent + 3 * (long)e + d) *
-             (__ldg(ev + (3 * (long)v0 + d) * K + c) + __ldg(ev + (3 * (long)v1 + d) * K + c));
-    val *= T(0.5);
-  } else {
-    T a = __ldg(ev + (long)v0 * K + c), b = __ldg(ev + (long)v1 * K + c);
-    if (sp == 0) val = b - a;
-    else val = T(0.5) * __ldg(tangent + 3 * (long)e + (sp - 1)) * (a + b);
+      for (int d = 0; d < 3; ++d) tg[d] = __ldg(tangent + 3 * e + d);
+    } else if (sp > 0) {
+      tg[0] = __ldg(tangent + 3 * e + (sp - 1));
+    }
   }
-  x[i] += val;
+  pdl_wait();
+  if (!valid) return;
+  const int c0 = (int)(t - e * cl) * V;
+  T xv[V], val[V], a[V], b[V];
+  ldv<T, V>(x + e * K + c0, xv);
+  if (sp == 4) {  // vector space: rows 3 v + d
+#pragma unroll
+    for (int i = 0; i < V; ++i) val[i] = T(0);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      ldv<T, V>(ev + (3 * (long)vv.x + d) * K + c0, a);
+      ldv<T, V>(ev + (3 * (long)vv.y + d) * K + c0, b);
+#pragma unroll
+      for (int i = 0; i < V; ++i) val[i] += tg[d] * (a[i] + b[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) val[i] *= T(0.5);
+  } else {
+    ldv<T, V>(ev + (long)vv.x * K + c0, a);
+    ldv<T, V>(ev + (long)vv.y * K + c0, b);
+#pragma unroll
+    for (int i = 0; i < V; ++i) val[i] = sp == 0 ? b[i] - a[i] : T(0.5) * tg[0] * (a[i] + b[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < V; ++i) xv[i] += val[i];
+  stv<T, V>(x + e * K + c0, xv);
 }
 
 template <typename T>
 void ams_prolong_add(int ne, int K, int sp, const int *edges, const T *tangent, const T *e_vert, T *x_edge,
                      cudaStream_t s) {
-  long total = (long)ne * K;
-  ams_prolong_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(ne, K, sp, edges, tangent, e_vert, x_edge);
+  if (ne <= 0) return;
+  const int v = vec_width<T>(K), cl = K / v;
+  const unsigned grid = (unsigned)(((long)ne * cl + 255) / 256);
+  if (v == 1) launch_chain(&ams_prolong_kernel<T, 1>, grid, 256, s, true, ne, K, cl, sp, edges, tangent, e_vert, x_edge);
+  else if (v == 2)
+    launch_chain(&ams_prolong_kernel<T, 2>, grid, 256, s, true, ne, K, cl, sp, edges, tangent, e_vert, x_edge);
+  else if constexpr (sizeof(T) == 4)
+    launch_chain(&ams_prolong_kernel<T, 4>, grid, 256, s, true, ne, K, cl, sp, edges, tangent, e_vert, x_edge);
   EMG_LAUNCH_CHECK();
 }
 
+// Dense coarsest solve: a warp per row and column pair, its lanes split the
+// row of the inverse (coalesced; up to kPre of its elements per lane load
+// before the wait), so a row is a handful of loads deep instead of nc.
 template <typename T>
-__global__ void coarse_apply_kernel(int nc, int K, const double *__restrict__ inv, const int *__restrict__ slot,
-                                    const T *__restrict__ b, T *__restrict__ x) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)nc * K) return;
-  int r = (int)(i / K), c = (int)(i % K);
-  const double *row = inv + ((long)__ldg(slot + c) * nc + r) * nc;
-  double acc = 0;
-  for (int j = 0; j < nc; ++j) acc += __ldg(row + j) * (double)b[(long)j * K + c];
-  x[i] = (T)acc;
+__global__ void __launch_bounds__(256) coarse_apply_kernel(int nc, int K, const double *__restrict__ inv,
+                                                           const int *__restrict__ slot, const T *b, T *x) {
+  constexpr int kPre = 8;
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, kp = (K + 1) / 2;
+  const int t = (int)((blockIdx.x * 256 + threadIdx.x) >> 5);
+  if (t >= nc * kp) {
+    pdl_wait();
+    return;
+  }
+  const int r = t / kp, c0 = (t - r * kp) * 2;
+  const bool pair = c0 + 1 < K;
+  const int s0 = __ldg(slot + c0), s1 = pair ? __ldg(slot + c0 + 1) : s0;
+  const double *row0 = inv + ((long)s0 * nc + r) * nc, *row1 = inv + ((long)s1 * nc + r) * nc;
+  double pre[kPre];
+#pragma unroll
+  for (int q = 0; q < kPre; ++q) pre[q] = lane + 32 * q < nc ? __ldg(row0 + lane + 32 * q) : 0.0;
+  pdl_wait();
+  double a0 = 0, a1 = 0;
+  auto add = [&](int j, double w0) {
+    const double w1 = s1 == s0 ? w0 : __ldg(row1 + j);
+    a0 += w0 * (double)b[(long)j * K + c0];
+    if (pair) a1 += w1 * (double)b[(long)j * K + c0 + 1];
+  };
+#pragma unroll
+  for (int q = 0; q < kPre; ++q)
+    if (lane + 32 * q < nc) add(lane + 32 * q, pre[q]);
+  for (int j = lane + 32 * kPre; j < nc; j += 32) add(j, __ldg(row0 + j));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+  }
+  if (lane == 0) {
+    x[(long)r * K + c0] = (T)a0;
+    if (pair) x[(long)r * K + c0 + 1] = (T)a1;
+  }
 }
 
 template <typename T>
 void coarse_apply(int nc, int K, const double *inv, const int *col_slot, const T *b, T *x, cudaStream_t s) {
-  long total = (long)nc * K;
-  if (!total) return;
-  coarse_apply_kernel<T><<<(unsigned)((total + 127) / 128), 128, 0, s>>>(nc, K, inv, col_slot, b, x);
+  if (nc <= 0) return;
+  const long warps = (long)nc * ((K + 1) / 2);
+  launch_chain(&coarse_apply_kernel<T>, (unsigned)((warps * 32 + 255) / 256), 256, s, true, nc, K, inv, col_slot, b, x);
   EMG_LAUNCH_CHECK();
 }
 
@@ -1035,11 +1177,11 @@ void abs_bound2(int n, int K, const int *rp, const int *ci, const double *Cv, co
                            cudaStream_t);                                                                        \
   template void fcg_update<T>(int, int, const double *, const T *, const T *, T *, T *, double *, cudaStream_t, float *); \
   template void fcg_direction<T>(int, int, const T *, int, T *const *, const double *, T *, cudaStream_t);       \
-  template void jacobi0<T>(int, int, const T *, const T *, const T *, const double *, double, T *, cudaStream_t); \
-  template void jacobi0_2<T>(int, int, const T *, const T *, const T *, const double *, double, T *, T *,           \
-                             cudaStream_t);                                                                      \
+  template void jacobi0<T>(int, int, const T *, const T *, const T *, const double *, double, T *, T *,          \
+                           cudaStream_t);                                                                        \
   template void fill_zero<T>(long, T *, cudaStream_t);                                                           \
-  template void ams_restrict<T>(int, int, int, const int *, const int *, const T *, const T *, T *, cudaStream_t); \
+  template void ams_restrict<T>(int, int, int, const int *, const int *, const T *, const T *, T *, cudaStream_t, \
+                                const RestrictJ0<T> &);                                                          \
   template void ams_prolong_add<T>(int, int, int, const int *, const T *, const T *, T *, cudaStream_t);          \
   template void coarse_apply<T>(int, int, const double *, const int *, const T *, T *, cudaStream_t);
 EMG_INST(float)

@@ -19,6 +19,8 @@
 
 #include <cstdint>
 
+#include "emg_pdl.cuh"
+
 namespace emg {
 
 enum SpmmMode : int {
@@ -40,6 +42,9 @@ enum SpmmMode : int {
   // (l1c/l1m of the args; d may be null), c1 = 1/theta (Chebyshev) or the
   // l1-Jacobi weight
   SPMM_AXJ0 = 7,
+  // the same for a right-hand side that is a residual: y = b - A x, r = d =
+  // c1 y / D' (A may have two parts)
+  SPMM_RESJ0 = 8,
 };
 
 template <typename T, int V>
@@ -50,17 +55,10 @@ template <> struct VecT<float, 4> { typedef float4 type; };
 template <> struct VecT<double, 1> { typedef double type; };
 template <> struct VecT<double, 2> { typedef double2 type; };
 
+// block vectors change within a chain of overlapping kernels: coherent loads,
+// never the read-only path
 template <typename T, int V>
-__device__ __forceinline__ void ldv(const T *__restrict__ p, T (&v)[V]) {
-  typedef typename VecT<T, V>::type VT;
-  VT t = __ldg(reinterpret_cast<const VT *>(p));
-  const T *s = reinterpret_cast<const T *>(&t);
-#pragma unroll
-  for (int i = 0; i < V; ++i) v[i] = s[i];
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void ldv_plain(const T *p, T (&v)[V]) {
+__device__ __forceinline__ void ldv(const T *p, T (&v)[V]) {
   typedef typename VecT<T, V>::type VT;
   VT t = *reinterpret_cast<const VT *>(p);
   const T *s = reinterpret_cast<const T *>(&t);
@@ -98,6 +96,9 @@ struct SpmmArgs {
   // row, values 0); row r owns chunks crp[r] .. crp[r+1]
   const int *crp;
   const int4 *ch;
+  // the launch may overlap its predecessor in the stream (emg_pdl.cuh): the
+  // operator, l1 sums and omega must be older than that predecessor
+  bool chained;
 };
 
 // One step of a fused nodal V-cycle (vcycle_fused_kernel): the operations a
@@ -116,38 +117,43 @@ struct FusedOp {
   SpmmArgs a;
 };
 
-// Row epilogue shared by the SpMM kernels, in two halves: epi_load reads
-// the row vectors the mode needs (b, x, r, y and the l1 sums; none of them
-// depends on the row product, so the kernels issue these loads before the
-// gathers and they overlap), epi_store combines them with the row product
-// acc (columns cb*V .. cb*V+V-1 of row `row`) and stores the results.
+// Row epilogue shared by the SpMM kernels, in three parts: epi_diag reads the
+// l1 sums the mode needs (older than the chain: before pdl_wait), epi_load the
+// row vectors (b, x, r, y; none of them depends on the row product, so the
+// kernels issue these loads before the gathers and they overlap), epi_store
+// combines them with the row product acc (columns cb*V .. cb*V+V-1 of row
+// `row`) and stores the results.
 template <typename T, int V>
 struct EpiIn {
   T b[V], x[V], r[V], y[V];
   T dc, dm;
 };
 
-template <typename T, int K, int V>
-__device__ __forceinline__ void epi_load(const SpmmArgs &a, int row, int cb, bool two, EpiIn<T, V> &e) {
-  const long o = (long)row * K + cb * V;
-  const T *__restrict__ x = static_cast<const T *>(a.x);
-  T *y = static_cast<T *>(a.y);
+template <typename T, int V>
+__device__ __forceinline__ void epi_diag(const SpmmArgs &a, int row, bool two, EpiIn<T, V> &e) {
   const int mode = a.mode;
-  const bool cheb = mode == SPMM_CHEB1 || mode == SPMM_CHEB2 || mode == SPMM_CHEBK;
-  // b of SPMM_CHEBK is r, which the same row overwrites: plain load
-  if (mode == SPMM_RES || mode == SPMM_JAC || mode == SPMM_CHEB1) ldv<T, V>(static_cast<const T *>(a.b) + o, e.b);
-  if (mode == SPMM_CHEBK) ldv_plain<T, V>(static_cast<const T *>(a.b) + o, e.b);
-  if (mode == SPMM_JAC || cheb) ldv<T, V>(x + o, e.x);
-  if (mode == SPMM_CHEB2) ldv<T, V>(static_cast<const T *>(a.r) + o, e.r);
-  if (mode == SPMM_ADD || mode == SPMM_CHEB2 || mode == SPMM_CHEBK) ldv_plain<T, V>(y + o, e.y);
-  if (mode == SPMM_JAC || cheb) {
+  if (mode == SPMM_JAC || mode == SPMM_CHEB1 || mode == SPMM_CHEB2 || mode == SPMM_CHEBK) {
     e.dc = __ldg(static_cast<const T *>(a.l1c) + row);
     e.dm = two ? __ldg(static_cast<const T *>(a.l1m) + row) : T(0);
   }
-  if (mode == SPMM_AXJ0) {  // the fed level's diagonal; A itself has one part
+  if (mode == SPMM_AXJ0 || mode == SPMM_RESJ0) {  // the fed level's diagonal
     e.dc = __ldg(static_cast<const T *>(a.l1c) + row);
     e.dm = a.l1m ? __ldg(static_cast<const T *>(a.l1m) + row) : T(0);
   }
+}
+
+template <typename T, int K, int V>
+__device__ __forceinline__ void epi_load(const SpmmArgs &a, int row, int cb, EpiIn<T, V> &e) {
+  const long o = (long)row * K + cb * V;
+  const T *x = static_cast<const T *>(a.x);
+  T *y = static_cast<T *>(a.y);
+  const int mode = a.mode;
+  const bool cheb = mode == SPMM_CHEB1 || mode == SPMM_CHEB2 || mode == SPMM_CHEBK;
+  if (mode == SPMM_RES || mode == SPMM_JAC || mode == SPMM_CHEB1 || mode == SPMM_CHEBK || mode == SPMM_RESJ0)
+    ldv<T, V>(static_cast<const T *>(a.b) + o, e.b);
+  if (mode == SPMM_JAC || cheb) ldv<T, V>(x + o, e.x);
+  if (mode == SPMM_CHEB2) ldv<T, V>(static_cast<const T *>(a.r) + o, e.r);
+  if (mode == SPMM_ADD || mode == SPMM_CHEB2 || mode == SPMM_CHEBK) ldv<T, V>(y + o, e.y);
 }
 
 template <typename T, int K, int V>
@@ -189,13 +195,14 @@ __device__ __forceinline__ void epi_store(const SpmmArgs &a, int row, int cb, co
     stv<T, V>(static_cast<T *>(a.d) + o, dd);
     break;
   }
-  case SPMM_AXJ0: {
+  case SPMM_AXJ0:
+  case SPMM_RESJ0: {
     T dd[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const T dg = a.l1m ? e.dc + (T)__ldg(a.omega + cb * V + i) * e.dm : e.dc;
-      out[i] = acc[i];
-      dd[i] = (T)a.c1 * acc[i] / dg;
+      out[i] = a.mode == SPMM_RESJ0 ? e.b[i] - acc[i] : acc[i];
+      dd[i] = (T)a.c1 * out[i] / dg;
     }
     stv<T, V>(static_cast<T *>(a.r) + o, dd);
     if (a.d) stv<T, V>(static_cast<T *>(a.d) + o, dd);
@@ -228,7 +235,8 @@ template <typename T, int K, int V>
 __device__ __forceinline__ void spmm_epilogue(const SpmmArgs &a, int row, int cb, const T (&acc)[V], const T (&w)[V],
                                               bool two) {
   EpiIn<T, V> e;
-  epi_load<T, K, V>(a, row, cb, two, e);
+  epi_diag<T, V>(a, row, two, e);
+  epi_load<T, K, V>(a, row, cb, e);
   epi_store<T, K, V>(a, row, cb, acc, w, two, e);
 }
 
@@ -239,6 +247,7 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   constexpr int CL = K / V;
   constexpr int G = NL * CL;
   static_assert(G <= 32 && (32 % G) == 0, "bad lane layout");
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int row = gwarp * (32 / G) + lane / G;
@@ -247,7 +256,7 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   const int sl = sub / CL;      // nonzero slice
   const T *__restrict__ vc = static_cast<const T *>(a.vc);
   const T *__restrict__ vm = static_cast<const T *>(a.vm);
-  const T *__restrict__ x = static_cast<const T *>(a.x);
+  const T *x = static_cast<const T *>(a.x);
   T acc[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = T(0);
@@ -257,46 +266,58 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   for (int i = 0; i < V; ++i) w[i] = two ? (T)__ldg(a.omega + cb * V + i) : T(0);
   const bool valid = row < a.n;
   EpiIn<T, V> epi;
-  if (valid && sl == 0) epi_load<T, K, V>(a, row, cb, two, epi);
+  int kb = 0, ke = 0;
   if (valid) {
-    const int kb = __ldg(a.rp + row), ke = __ldg(a.rp + row + 1);
-    // U nonzeros per lane per round: all index/value loads of the round are
-    // issued before the dependent x gathers, so U gathers are in flight at
-    // once (rows are short, ~16 nonzeros, and split NL ways)
-    constexpr int U = 4;
-    for (int k0 = kb + sl; k0 < ke; k0 += NL * U) {
-      int j[U];
-      T c[U], m[U];
-      bool ok[U];
+    kb = __ldg(a.rp + row);
+    ke = __ldg(a.rp + row + 1);
+  }
+  // U nonzeros per lane per round: all index/value loads of the round are
+  // issued before the dependent x gathers, so U gathers are in flight at
+  // once (rows are short, ~16 nonzeros, and split NL ways)
+  constexpr int U = 4;
+  int k0 = kb + sl;
+  int j[U];
+  T c[U], m[U];
+  bool ok[U];
+  auto fetch = [&]() {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = k0 + u * NL;
-        ok[u] = k < ke;
-        if constexpr (PK) {
-          const int4 rec = ok[u] ? __ldg(a.pk + k) : make_int4(0, 0, 0, 0);
-          j[u] = rec.x;
-          c[u] = (T)__int_as_float(rec.y);
-          m[u] = (T)__int_as_float(rec.z);
-        } else {
-          j[u] = ok[u] ? __ldg(a.ci + k) : 0;
-          c[u] = ok[u] ? __ldg(vc + k) : T(0);
-          m[u] = (ok[u] && two) ? __ldg(vm + k) : T(0);
-        }
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * NL;
+      ok[u] = k < ke;
+      if constexpr (PK) {
+        const int4 rec = ok[u] ? __ldg(a.pk + k) : make_int4(0, 0, 0, 0);
+        j[u] = rec.x;
+        c[u] = (T)__int_as_float(rec.y);
+        m[u] = (T)__int_as_float(rec.z);
+      } else {
+        j[u] = ok[u] ? __ldg(a.ci + k) : 0;
+        c[u] = ok[u] ? __ldg(vc + k) : T(0);
+        m[u] = (ok[u] && two) ? __ldg(vm + k) : T(0);
       }
-      T xv[U][V];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (ok[u]) ldv<T, V>(x + (long)j[u] * K + cb * V, xv[u]);
-        else {
-#pragma unroll
-          for (int i = 0; i < V; ++i) xv[u][i] = T(0);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] = fma(two ? c[u] + w[i] * m[u] : c[u], xv[u][i], acc[i]);
     }
+  };
+  // the first round of the matrix before the wait: on the small levels that
+  // is the whole row, and only the gathers remain of the dependent chain
+  fetch();
+  if (valid && sl == 0) epi_diag<T, V>(a, row, two, epi);
+  pdl_wait();
+  if (valid && sl == 0) epi_load<T, K, V>(a, row, cb, epi);
+  while (k0 < ke) {
+    T xv[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (ok[u]) ldv<T, V>(x + (long)j[u] * K + cb * V, xv[u]);
+      else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) xv[u][i] = T(0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] = fma(two ? c[u] + w[i] * m[u] : c[u], xv[u][i], acc[i]);
+    k0 += NL * U;
+    if (k0 < ke) fetch();
   }
 #pragma unroll
   for (int off = CL; off < G; off <<= 1)
@@ -324,10 +345,12 @@ __global__ void __launch_bounds__(256) spmm_pipe_kernel(SpmmArgs a) {
   const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int row = gwarp * (32 / CL) + lane / CL;
   const int cb = lane % CL;
+  pdl_trigger();
+  pdl_wait();
   if (row >= a.n) return;
   const T *__restrict__ vc = static_cast<const T *>(a.vc);
   const T *__restrict__ vm = static_cast<const T *>(a.vm);
-  const T *__restrict__ x = static_cast<const T *>(a.x);
+  const T *x = static_cast<const T *>(a.x);
   const bool two = vm != nullptr;
   T w[V], acc[V];
 #pragma unroll
@@ -336,7 +359,8 @@ __global__ void __launch_bounds__(256) spmm_pipe_kernel(SpmmArgs a) {
     acc[i] = T(0);
   }
   EpiIn<T, V> epi;
-  epi_load<T, K, V>(a, row, cb, two, epi);
+  epi_diag<T, V>(a, row, two, epi);
+  epi_load<T, K, V>(a, row, cb, epi);
   const int kb = __ldg(a.rp + row), ke = __ldg(a.rp + row + 1);
   int j[U];
   T c[U], m[U];
@@ -392,7 +416,7 @@ __global__ void __launch_bounds__(256) spmm_pipe_kernel(SpmmArgs a) {
 template <bool PAIRS, int K, int V>
 __device__ __forceinline__ void chunk_rows(const SpmmArgs &a, int q0, int q1, int cb, const float (&w)[V],
                                            float (&acc)[V]) {
-  const float *__restrict__ xb = static_cast<const float *>(a.x) + cb * V;
+  const float *xb = static_cast<const float *>(a.x) + cb * V;
   for (int q = q0; q < q1; ++q) {
     const int4 jj = __ldg(a.ch + 3 * q);
     const int4 cr = __ldg(a.ch + 3 * q + 1);
@@ -428,7 +452,11 @@ __global__ void __launch_bounds__(256, MINB) spmm_chunk_kernel(SpmmArgs a) {
   const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int row = gwarp * (32 / CL) + lane / CL;
   const int cb = lane % CL;
-  if (row >= a.n) return;  // no shuffles: a lane past the end leaves at once
+  pdl_trigger();
+  if (row >= a.n) {  // no shuffles: a lane past the end leaves
+    pdl_wait();
+    return;
+  }
   float w[V], acc[V];
   bool pairs = (V % 2) == 0;
 #pragma unroll
@@ -439,8 +467,10 @@ __global__ void __launch_bounds__(256, MINB) spmm_chunk_kernel(SpmmArgs a) {
 #pragma unroll
   for (int i = 0; i + 1 < V; i += 2) pairs = pairs && w[i] == w[i + 1];
   EpiIn<float, V> epi;
-  epi_load<float, K, V>(a, row, cb, true, epi);
   const int q0 = __ldg(a.crp + row), q1 = __ldg(a.crp + row + 1);
+  epi_diag<float, V>(a, row, true, epi);
+  pdl_wait();
+  epi_load<float, K, V>(a, row, cb, epi);
   if (pairs) chunk_rows<true, K, V>(a, q0, q1, cb, w, acc);
   else chunk_rows<false, K, V>(a, q0, q1, cb, w, acc);
   epi_store<float, K, V>(a, row, cb, acc, w, true, epi);
@@ -458,6 +488,7 @@ __global__ void __launch_bounds__(256) spmm_rows_kernel(SpmmArgs a) {
   constexpr int G = K / V;
   constexpr int RPW = 32 / G;
   static_assert(G <= 32 && (32 % G) == 0 && (G % B) == 0, "bad row-group layout");
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int grp = lane / G, j = lane % G;
@@ -465,7 +496,7 @@ __global__ void __launch_bounds__(256) spmm_rows_kernel(SpmmArgs a) {
   const bool valid = row < a.n;
   const T *__restrict__ vc = static_cast<const T *>(a.vc);
   const T *__restrict__ vm = static_cast<const T *>(a.vm);
-  const T *__restrict__ x = static_cast<const T *>(a.x);
+  const T *x = static_cast<const T *>(a.x);
   const bool two = vm != nullptr;
   T w[V], acc[V];
 #pragma unroll
@@ -476,7 +507,9 @@ __global__ void __launch_bounds__(256) spmm_rows_kernel(SpmmArgs a) {
   const int kb = valid ? __ldg(a.rp + row) : 0;
   const int len = valid ? __ldg(a.rp + row + 1) - kb : 0;
   EpiIn<T, V> epi;
-  if (valid) epi_load<T, K, V>(a, row, j, two, epi);
+  if (valid) epi_diag<T, V>(a, row, two, epi);
+  pdl_wait();
+  if (valid) epi_load<T, K, V>(a, row, j, epi);
   int maxlen = len;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, off));
@@ -532,13 +565,15 @@ __global__ void __launch_bounds__(256) spmm_tiled_kernel(SpmmArgs a, TiledArgs t
   constexpr int CL = K / V;     // lanes over the columns of one row
   constexpr int RPW = 32 / CL;  // rows per warp
   static_assert(CL <= 32 && (32 % CL) == 0, "bad tiled lane layout");
+  pdl_trigger();
   const int tile = blockIdx.x;
   const int u0 = __ldg(t.urp + tile), nu = __ldg(t.urp + tile + 1) - u0;
-  const T *__restrict__ x = static_cast<const T *>(a.x);
+  const T *x = static_cast<const T *>(a.x);
+  pdl_wait();
   for (int idx = threadIdx.x; idx < nu * CL; idx += blockDim.x) {
     const int u = idx / CL, cb = idx - u * CL;
     const long g = __ldg(t.ucol + u0 + u);
-    *reinterpret_cast<VT *>(xs + u * K + cb * V) = __ldg(reinterpret_cast<const VT *>(x + g * K + cb * V));
+    *reinterpret_cast<VT *>(xs + u * K + cb * V) = *reinterpret_cast<const VT *>(x + g * K + cb * V);
   }
   __syncthreads();
   const T *__restrict__ vc = static_cast<const T *>(a.vc);

@@ -73,14 +73,10 @@ void fcg_update(int n, int K, const double *alpha, const T *p, const T *sv, T *x
 // p = z - sum_j beta[j*K+c] * P_j  (nprev directions, pointers in a device array)
 template <typename T>
 void fcg_direction(int n, int K, const T *z, int nprev, T *const *Pj, const double *beta, T *p, cudaStream_t st);
-// y = w * b / d   (first l1-Jacobi sweep from a zero guess)
+// y (and d when given) = w * b / D  (first smoothing step from a zero guess)
 template <typename T>
-void jacobi0(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y,
+void jacobi0(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y, T *d,
              cudaStream_t s);
-// y = d = w * b / D  (first smoothing step from a zero guess, two outputs)
-template <typename T>
-void jacobi0_2(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y, T *d,
-               cudaStream_t s);
 // precision conversion of block vectors
 void cvt_d2f(long count, const double *a, float *b, cudaStream_t s);
 void cvt_f2d(long count, const float *a, double *b, cudaStream_t s);
@@ -103,9 +99,18 @@ void zsplit_direction(int n, int K, const int *edges, const float *x, const floa
 //   sp == 0: gradient G (row e: -1 at edges[e][0], +1 at edges[e][1])
 //   sp == 1..3: Pi_d, d = sp-1 (row e: 0.5 t_e[d] at both endpoints)
 //   sp == 4: Pi = [Pi_x Pi_y Pi_z], vertex vectors stored as rows 3 v + d
+// With j0.y the restriction also takes the first zero-guess smoothing step of
+// the level it feeds: y = d = c1 r_vert / (l1c + w_c l1m).
+template <typename T>
+struct RestrictJ0 {
+  const T *l1c, *l1m;
+  const double *omega;
+  double c1;
+  T *y, *d;
+};
 template <typename T>
 void ams_restrict(int nv, int K, int sp, const int *inc_rp, const int *inc, const T *tangent, const T *r_edge,
-                  T *r_vert, cudaStream_t s);
+                  T *r_vert, cudaStream_t s, const RestrictJ0<T> &j0 = RestrictJ0<T>{});
 template <typename T>
 void ams_prolong_add(int ne, int K, int sp, const int *edges, const T *tangent, const T *e_vert, T *x_edge,
                      cudaStream_t s);

@@ -512,6 +512,7 @@ void Ams<T>::spmm_B(int mode, const T *x, const T *b, T *y, cudaStream_t s) {
   a.y = y;
   a.relax_w = relax_w;
   a.mode = mode;
+  a.chained = true;
   KernelProfiler &pf = profiler();
   cudaEvent_t ev = nullptr;
   const char *bin = sizeof(T) == 4 ? "spmm_edge_fp32" : "spmm_edge_fp64";
@@ -568,8 +569,7 @@ void Ams<T>::emit_jac0(int n, const T *b, const T *l1c, const T *l1m, double w, 
     rec->push_back(op);
     return;
   }
-  if (d) jacobi0_2<T>(n, K, b, l1c, l1m, omega.p, w, y, d, s);
-  else jacobi0<T>(n, K, b, l1c, l1m, omega.p, w, y, s);
+  jacobi0<T>(n, K, b, l1c, l1m, omega.p, w, y, d, s);
 }
 
 template <typename T>
@@ -609,6 +609,7 @@ static SpmmArgs level_args(const DCsr<T> &A, int mode, const double *omega, doub
   a.y = y;
   a.relax_w = w;
   a.mode = mode;
+  a.chained = true;
   return a;
 }
 
@@ -671,6 +672,7 @@ T *Ams<T>::smooth(const DCsr<T> *A, long nnz, int n, T *cur, T *oth, const T *b,
     a.d = d;
     a.c1 = c1;
     a.c2 = c2;
+    a.chained = true;
     emit_spmm(a, nnz, bin, s, edge ? edge_tiles() : nullptr);
   };
   if (!cheb) {
@@ -833,9 +835,20 @@ void Ams<T>::check_fused(cudaStream_t s) {
 }
 
 template <typename T>
-void Ams<T>::run_vcycle(int sp, cudaStream_t s) {
+void Ams<T>::run_vcycle(int sp, cudaStream_t s, bool started) {
   if (fused && (fused_epoch != graphs.epoch || ws_K != K)) prepare_fused(s);
-  vcycle(sp, 0, s);
+  vcycle(sp, 0, s, started);
+}
+
+template <typename T>
+bool Ams<T>::start_step(int sp, RestrictJ0<T> &j0) {
+  const Sub &S = sub[sp];
+  if (!restrict_j0 || !amg_pre_smooth || fused || S.lv.empty()) return false;
+  const int swaps = 2 * amg_relax_times - 1;  // as vcycle(): the buffer its smoothing starts in
+  const DCsr<T> &A = S.lv[0].A;
+  j0 = RestrictJ0<T>{A.l1c.p, A.l1m.p, omega.p, cheb ? cheb_coef(amg_cheb_degree).inv_theta : relax_w,
+                     (swaps & 1) ? wx2[sp][0].p : wx[sp][0].p, cheb ? wd[sp][0].p : nullptr};
+  return true;
 }
 
 template <typename T>
@@ -930,11 +943,13 @@ void Ams<T>::apply_eager(const T *b, T *x, cudaStream_t s) {
     const int sp = ams_subspace(ch);
     if (sp < 0) fail(EMG_ERR_OPTION, "bad AMS cycle character '%c'", ch);
     const T *tg = sp == 0 ? nullptr : tangent.p;
+    RestrictJ0<T> j0{};
+    const bool started = start_step(sp, j0);
     if (sp == 0) {
       // gradient space: G^T (b - B x) = G^T b - (G^T B) x
       if (zero) {
         fill_zero<T>((long)ne * K, cur, s);
-        ams_restrict<T>(nv, K, 0, inc_rp, inc, nullptr, b, wb[0][0].p, s);
+        ams_restrict<T>(nv, K, 0, inc_rp, inc, nullptr, b, wb[0][0].p, s, j0);
         zero = false;
       } else {
         ams_restrict<T>(nv, K, 0, inc_rp, inc, nullptr, b, gtmp.p, s);
@@ -945,15 +960,19 @@ void Ams<T>::apply_eager(const T *b, T *x, cudaStream_t s) {
         a.ci = gci;
         a.vc = gvc.p;
         a.vm = two ? (const void *)gvm.p : nullptr;
-        a.l1c = a.l1m = nullptr;
+        a.l1c = j0.l1c;
+        a.l1m = j0.l1m;
         a.omega = omega.p;
         a.x = cur;
         a.b = gtmp.p;
         a.y = wb[0][0].p;
         a.relax_w = 1.0;
-        a.mode = SPMM_RES;
-        a.r = a.d = nullptr;
-        a.c1 = a.c2 = 0;
+        a.mode = started ? SPMM_RESJ0 : SPMM_RES;
+        a.r = j0.y;
+        a.d = j0.d;
+        a.c1 = j0.c1;
+        a.c2 = 0;
+        a.chained = true;
         const TiledPattern *tp = gtb_tiles();
         if (tp) spmm_tiled<T>(K, a, *tp, s);
         else spmm_nnz<T>(K, a, nnzG, s);
@@ -966,9 +985,9 @@ void Ams<T>::apply_eager(const T *b, T *x, cudaStream_t s) {
       } else {
         spmm_B(SPMM_RES, cur, b, er.p, s);
       }
-      ams_restrict<T>(nv, K, sp, inc_rp, inc, tg, er.p, wb[sp][0].p, s);
+      ams_restrict<T>(nv, K, sp, inc_rp, inc, tg, er.p, wb[sp][0].p, s, j0);
     }
-    run_vcycle(sp, s);
+    run_vcycle(sp, s, started);
     // split form: the closing gradient correction stays a vertex potential
     // (wx[0][0]); the caller adds G phi in higher precision
     if (split_gradient && sp == 0 && ci + 1 == cycle.size()) continue;

@@ -170,7 +170,11 @@ struct Ams {
   void vcycle(int sp, int l, cudaStream_t s, bool started = false);
   // runs subspace sp's V-cycle: the levels with at least fused_rows rows
   // step by step, the rest as one fused launch
-  void run_vcycle(int sp, cudaStream_t s);
+  // (started: as vcycle)
+  void run_vcycle(int sp, cudaStream_t s, bool started = false);
+  // whether the restriction into subspace sp's finest level takes its first
+  // smoothing step, and with what
+  bool start_step(int sp, RestrictJ0<T> &j0);
   void launch_fused(int sp, cudaStream_t s);
   // records the fused step lists for the current workspace (not while capturing)
   void prepare_fused(cudaStream_t s);

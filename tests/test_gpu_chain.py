@@ -1,0 +1,66 @@
+"""The AMS chain at every block width, against a sparse direct solve.
+
+The transfers, first smoothing steps, coarsest solve and SpMMs of the AMS run
+as overlapping kernels (programmatic dependent launch) whose lane layout
+follows the block width: 1, 2 or 4 columns per load, 1 to 4 lanes per row or
+vertex, padded blocks.  Each width solves CSEM right-hand sides on a mesh of
+some 1000 cells; the solutions must agree with the direct solve to 1e-6 of
+the largest value per column, the bar of the other solve tests (rtol 1e-8, a
+factor 100 for the condition between residual and error at 0.5-4 Hz).
+"""
+
+import numpy as np
+import pytest
+
+import emfem_b200 as E
+from emfem_b200 import meshgen as mg
+from exact_solve import exact_solutions
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def system():
+    import torch
+    freqs = np.array([0.5, 4.0])
+    prob = mg.marine_csem(1200, freqs=freqs, n_tx=3, name="chain")
+    c = E.EMContext(0)
+    c.set_mesh(prob.mesh)
+    c.set_model(prob.model)
+    c.set_frequencies(freqs)
+    c.create_linear_system(0)
+    rp, ci = c.make_sparsity_patterns()
+    ne = prob.mesh.n_edges
+    tx = np.tile(prob.survey.tx, (2, 1))
+    colf = np.repeat(freqs, 3)
+    s = torch.zeros((ne, 6), dtype=torch.complex128, device="cuda")
+    c.assemble_matrix(0)
+    c.assemble_rhs_csem_block_dev(colf, tx, s.data_ptr())
+    s = s.cpu().numpy()
+    jobs = []
+    for f in range(2):
+        c.assemble_matrix(f)
+        Cv, Mv, _ = c.get_matrices()
+        jobs.append((rp, ci, Cv, Mv, np.conj(s[:, 3 * f:3 * f + 3])))
+    exact = np.concatenate(exact_solutions(jobs), axis=1)
+    yield c, colf, s, exact
+    c.close()
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 8, 17])
+@pytest.mark.parametrize("options", ["-emg_restrict_smooth 1 -emg_smoother chebyshev",
+                                     "-emg_restrict_smooth 0 -emg_smoother chebyshev",
+                                     "-emg_restrict_smooth 1 -emg_smoother l1jacobi"])
+def test_block_widths(system, fp32, k, options):
+    c, colf, s, exact = system
+    if "l1jacobi" in options and k != 3:
+        pytest.skip("one width per smoother")
+    cols = np.arange(k) % 6
+    # coarsest grids small enough that the hierarchy has several levels
+    c.process_options("-emg_amg_max_coarse 40 " + options)
+    c.assemble_matrix(0)
+    x, infos = c.solve_block(colf[cols], s[:, cols], rtol=1e-8, max_it=200, inner_fp32=fp32)
+    assert all(i.reason == 0 for i in infos)
+    err = np.abs(x - exact[:, cols]).max(axis=0) / np.abs(exact[:, cols]).max(axis=0)
+    assert err.max() <= 1e-6, err
