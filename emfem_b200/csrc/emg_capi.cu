@@ -110,8 +110,7 @@ void launch_rhs_mt(Context &c, int k, const double *omega_dev, const double *bv_
                    double *s_dev);
 
 struct Workspace {
-  Fcg<double> fcg64;
-  Fcg<float> fcg32;
+  Fcg fcg64;
   Fgmres gm;
   DBuf<double> vec_a, vec_b;       // host<->device staging of complex block vectors
   DBuf<float> f_in, f_out;         // FP32 inner vectors
@@ -125,7 +124,7 @@ struct Workspace {
   Ams<double> bams64;
   Ams<float> bams32;
   // divergence correction of the batched path
-  Fcg<double> fcg_div;
+  Fcg fcg_div;
   DBuf<double> div_d, div_dis, div_ds;          // nv: l1 scale, its -1/2 and 1/2 powers (0 on the boundary)
   DBuf<double> div_rhs, div_y, div_t, div_u;    // nv x K2
   DBuf<double> div_e, div_me;                   // ne x K2
@@ -938,7 +937,7 @@ int emg_pc_apply_b(emg_context *c, const double *b, double *x) {
   w.vec_b.alloc((size_t)n * 2);
   w.fcg64.mmax = c->opt.fcg_mmax;
   w.fcg64.check_every = 1;
-  w.fcg64.solve(w.pams64, w.vec_a.p, w.vec_b.p, c->opt.inner_rtol, c->opt.inner_max_it, c->stream);
+  fcg_solve(w.fcg64, w.pams64, w.vec_a.p, w.vec_b.p, c->opt.inner_rtol, c->opt.inner_max_it, c->stream);
   std::vector<double> xo((size_t)n * 2);
   w.vec_b.download(xo.data(), xo.size(), c->stream);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
@@ -982,7 +981,7 @@ int emg_solve_linear_system(emg_context *c, int target, const double *s_re, cons
   w.fcg64.total_its = 0;
   SolveStats st;
   auto pc = [&](const double *v, double *z) {
-    w.fcg64.solve(w.pams64, v, z, c->opt.inner_rtol, c->opt.inner_max_it, c->stream);
+    fcg_solve(w.fcg64, w.pams64, v, z, c->opt.inner_rtol, c->opt.inner_max_it, c->stream);
   };
   w.gm.solve(*c, w.vec_a.p, x.p, false, rtol, max_it, true, pc, st);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1440,8 +1439,6 @@ static long div_correct(Context &c, int k, bool fp32, const double *b, double *x
   // scaled preconditioner: D^1/2 V D^1/2 with V the gradient space's V-cycle
   auto pc = [&](const double *r_, double *z_) {
     if (fp32) {
-      w.div_tf.alloc(NV);
-      w.div_uf.alloc(NV);
       vrow_scale<double, float>(nv, K2, w.div_ds.p, r_, w.div_tf.p, s);
       w.bams32.grad_vcycle(w.div_tf.p, w.div_uf.p, s);
       vrow_scale<float, double>(nv, K2, w.div_ds.p, w.div_uf.p, z_, s);
@@ -1455,7 +1452,26 @@ static long div_correct(Context &c, int k, bool fp32, const double *b, double *x
   w.fcg_div.check_every = c.opt.block_fcg_check_every;
   w.fcg_div.verbose = c.opt.verbose > 1;
   w.fcg_div.total_its = 0;
-  w.fcg_div.solve_with(nv, K2, pc, op, w.div_rhs.p, w.div_y.p, c.opt.div_rtol, c.opt.div_max_it, s);
+  std::vector<uint64_t> sig;
+  {
+    const KernelProfiler &pf = profiler();
+    const bool graphs = fp32 ? w.bams32.use_graphs && !w.bams32.fused : w.bams64.use_graphs && !w.bams64.fused;
+    if (fp32) {
+      w.div_tf.alloc(NV);
+      w.div_uf.alloc(NV);
+    }
+    if (graphs && !pf.enabled && !pf.phases) {
+      if (fp32) w.bams32.signature(sig);
+      else w.bams64.signature(sig);
+      for (const void *p : {(const void *)c.Msv.p, (const void *)c.rp.p, (const void *)c.ci.p, (const void *)omega,
+                            (const void *)c.edges.p, (const void *)c.vinc_rp.p, (const void *)c.vinc.p,
+                            (const void *)w.div_dis.p, (const void *)w.div_ds.p, (const void *)w.div_t.p,
+                            (const void *)w.div_u.p, (const void *)w.div_e.p, (const void *)w.div_me.p,
+                            (const void *)w.div_tf.p, (const void *)w.div_uf.p})
+        sig.push_back((uint64_t)p);
+    }
+  }
+  w.fcg_div.solve(nv, K2, pc, op, w.div_rhs.p, w.div_y.p, c.opt.div_rtol, c.opt.div_max_it, s, FcgFeed{}, nullptr, sig);
   // x += G D^-1/2 y
   vrow_scale<double, double>(nv, K2, w.div_dis.p, w.div_y.p, w.div_t.p, s);
   ams_prolong_add<double>(ne, K2, 0, c.edges.p, nullptr, w.div_t.p, x, s);
@@ -1506,10 +1522,10 @@ static void solve_block_pow2(Context &c, int k, const double *freqs, const doubl
   w.gm.stall_factor = (fp32 && c.opt.block_fp64_fallback) ? 0.5 : 0.0;
   w.gm.floor_stop = c.opt.block_floor_stop != 0;
   w.gm.omega.upload(om, c.stream);
-  w.fcg64.mmax = w.fcg32.mmax = c.opt.block_fcg_mmax;
-  w.fcg64.check_every = w.fcg32.check_every = c.opt.block_fcg_check_every;
-  w.fcg64.verbose = w.fcg32.verbose = c.opt.verbose > 1;
-  w.fcg64.total_its = w.fcg32.total_its = 0;
+  w.fcg64.mmax = c.opt.block_fcg_mmax;
+  w.fcg64.check_every = c.opt.block_fcg_check_every;
+  w.fcg64.verbose = c.opt.verbose > 1;
+  w.fcg64.total_its = 0;
   if (fp32) {
     w.f_in.alloc((size_t)n * k * 2);
     w.f_out.alloc((size_t)n * k * 2);
@@ -1547,28 +1563,38 @@ static void solve_block_pow2(Context &c, int k, const double *freqs, const doubl
     if (pf.enabled) pf.end("spmm_edge_fp64", c.stream, ev);
     if (pf.phases) pf.end("phase_opB", c.stream, ph);
   };
+  FcgFeed feed;
   auto pc32 = [&](const double *r_, double *z_) {
     KernelProfiler &pf = profiler();
     cudaEvent_t ph = nullptr;
     if (pf.phases) pf.begin("phase_ams", c.stream, 0, &ph);
     (void)r_;  // w.f_in holds (float) r_: the FCG update writes it
     (void)z_;  // z = f_out + G gphi is formed inside the FCG's passes
-    w.bams32.apply(w.f_in.p, w.f_out.p, c.stream);
+    w.bams32.apply(w.f_in.p, w.f_out.p, c.stream, feed.jf.y != nullptr);
     if (pf.phases) pf.end("phase_ams", c.stream, ph);
   };
-  Fcg<double>::ZSplit zsplit{c.edges.p, nullptr, nullptr};
+  Fcg::ZSplit zsplit{c.edges.p, nullptr, nullptr};
   auto pc = [&](const double *v, double *z) {
     KernelProfiler &pf = profiler();
     cudaEvent_t ph = nullptr;
     if (pf.phases) pf.begin("phase_fcg", c.stream, 0, &ph);
     if (fp32) {
       if (w.fcg64.mmax > 4) fail(EMG_ERR_OPTION, "-emg_block_fcg_mmax above 4 with the FP32 preconditioner");
+      feed.r32 = w.f_in.p;
+      feed.jf = w.bams32.edge_start(w.f_out.p);
+      std::vector<uint64_t> sig;
+      if (w.bams32.use_graphs && !w.bams32.fused && !pf.enabled && !pf.phases) {
+        w.bams32.signature(sig);
+        for (const void *p : {(const void *)c.Cv.p, (const void *)c.Msv.p, (const void *)c.rp.p, (const void *)c.ci.p,
+                              (const void *)w.omega_cols.p, (const void *)w.f_in.p, (const void *)w.f_out.p})
+          sig.push_back((uint64_t)p);
+      }
       zsplit.x = w.f_out.p;
       zsplit.phi = w.bams32.gphi();
-      w.fcg64.solve_with(n, K2, pc32, opB64, v, z, c.opt.block_inner_rtol, c.opt.block_inner_max_it, c.stream,
-                         w.f_in.p, &zsplit);
+      w.fcg64.solve(n, K2, pc32, opB64, v, z, c.opt.block_inner_rtol, c.opt.block_inner_max_it, c.stream, feed,
+                    &zsplit, sig);
     }
-    else w.fcg64.solve(w.bams64, v, z, c.opt.block_inner_rtol, c.opt.block_inner_max_it, c.stream);
+    else fcg_solve(w.fcg64, w.bams64, v, z, c.opt.block_inner_rtol, c.opt.block_inner_max_it, c.stream);
     if (pf.phases) pf.end("phase_fcg", c.stream, ph);
   };
   SolveStats st;

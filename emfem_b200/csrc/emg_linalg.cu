@@ -420,120 +420,6 @@ static unsigned red_grid(long total) {
   return (unsigned)std::max(1L, std::min(g, 148L * 8));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) coldot_kernel(long total, int K, const T *__restrict__ a,
-                                                     const T *__restrict__ b, double *__restrict__ out) {
-  __shared__ double sh[256];
-  double acc = 0;
-  for (long i = blockIdx.x * 256L + threadIdx.x; i < total; i += (long)gridDim.x * 256)
-    acc += (double)a[i] * (double)b[i];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = 128; st >= K; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if ((int)threadIdx.x < K) atomicAdd(out + threadIdx.x, sh[threadIdx.x]);
-}
-
-template <typename T>
-void coldot(int n, int K, const T *a, const T *b, double *out, cudaStream_t s) {
-  long total = (long)n * K;
-  coldot_kernel<T><<<red_grid(total), 256, 0, s>>>(total, K, a, b, out);
-  EMG_LAUNCH_CHECK();
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) coldot3_kernel(long total, int K, const T *__restrict__ a1,
-                                                      const T *__restrict__ b1, const T *__restrict__ a2,
-                                                      const T *__restrict__ b2, const T *__restrict__ a3,
-                                                      const T *__restrict__ b3, double *__restrict__ out) {
-  __shared__ double sh[3][256];
-  double s1 = 0, s2 = 0, s3 = 0;
-  for (long i = blockIdx.x * 256L + threadIdx.x; i < total; i += (long)gridDim.x * 256) {
-    s1 += (double)a1[i] * (double)b1[i];
-    s2 += (double)a2[i] * (double)b2[i];
-    if (a3) s3 += (double)a3[i] * (double)b3[i];
-  }
-  sh[0][threadIdx.x] = s1;
-  sh[1][threadIdx.x] = s2;
-  sh[2][threadIdx.x] = s3;
-  __syncthreads();
-  for (int st = 128; st >= K; st >>= 1) {
-    if ((int)threadIdx.x < st) {
-      sh[0][threadIdx.x] += sh[0][threadIdx.x + st];
-      sh[1][threadIdx.x] += sh[1][threadIdx.x + st];
-      sh[2][threadIdx.x] += sh[2][threadIdx.x + st];
-    }
-    __syncthreads();
-  }
-  if ((int)threadIdx.x < K) {
-    atomicAdd(out + threadIdx.x, sh[0][threadIdx.x]);
-    atomicAdd(out + K + threadIdx.x, sh[1][threadIdx.x]);
-    if (a3) atomicAdd(out + 2 * K + threadIdx.x, sh[2][threadIdx.x]);
-  }
-}
-
-template <typename T>
-void coldot3(int n, int K, const T *a1, const T *b1, const T *a2, const T *b2, const T *a3, const T *b3,
-             double *out, cudaStream_t s) {
-  long total = (long)n * K;
-  coldot3_kernel<T><<<red_grid(total), 256, 0, s>>>(total, K, a1, b1, a2, b2, a3, b3, out);
-  EMG_LAUNCH_CHECK();
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) fcg_update_kernel(long total, int K, const double *__restrict__ alpha,
-                                                         const T *__restrict__ p, const T *__restrict__ sv,
-                                                         T *__restrict__ x, T *__restrict__ r,
-                                                         double *__restrict__ rn, float *__restrict__ r32) {
-  __shared__ double sh[256];
-  double acc = 0;
-  const int c = threadIdx.x % K;
-  const double al = alpha[c];
-  for (long i = blockIdx.x * 256L + threadIdx.x; i < total; i += (long)gridDim.x * 256) {
-    T xi = x[i] + (T)al * p[i];
-    T ri = r[i] - (T)al * sv[i];
-    x[i] = xi;
-    r[i] = ri;
-    if (r32) r32[i] = (float)ri;
-    acc += (double)ri * (double)ri;
-  }
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = 128; st >= K; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if ((int)threadIdx.x < K) atomicAdd(rn + threadIdx.x, sh[threadIdx.x]);
-}
-
-template <typename T>
-void fcg_update(int n, int K, const double *alpha, const T *p, const T *sv, T *x, T *r, double *rn,
-                cudaStream_t s, float *r32) {
-  long total = (long)n * K;
-  fcg_update_kernel<T><<<red_grid(total), 256, 0, s>>>(total, K, alpha, p, sv, x, r, rn, r32);
-  EMG_LAUNCH_CHECK();
-}
-
-template <typename T>
-__global__ void fcg_direction_kernel(long total, int K, const T *__restrict__ z, int nprev, T *const *Pj,
-                                     const double *__restrict__ beta, T *__restrict__ p) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  int c = (int)(i % K);
-  double v = (double)z[i];
-  for (int j = 0; j < nprev; ++j) v -= beta[j * K + c] * (double)Pj[j][i];
-  p[i] = (T)v;
-}
-
-template <typename T>
-void fcg_direction(int n, int K, const T *z, int nprev, T *const *Pj, const double *beta, T *p, cudaStream_t st) {
-  long total = (long)n * K;
-  fcg_direction_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(total, K, z, nprev, Pj, beta, p);
-  EMG_LAUNCH_CHECK();
-}
-
 // columns per vector load of a K-column block row
 template <typename T>
 static int vec_width(int K) {
@@ -584,99 +470,11 @@ __global__ void cvt_d2f_kernel(long n, const double *__restrict__ a, float *__re
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)a[i];
 }
-__global__ void cvt_f2d_kernel(long n, const float *__restrict__ a, double *__restrict__ b) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (double)a[i];
-}
 void cvt_d2f(long count, const double *a, float *b, cudaStream_t s) {
   if (!count) return;
   cvt_d2f_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(count, a, b);
   EMG_LAUNCH_CHECK();
 }
-void cvt_f2d(long count, const float *a, double *b, cudaStream_t s) {
-  if (!count) return;
-  cvt_f2d_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(count, a, b);
-  EMG_LAUNCH_CHECK();
-}
-__global__ void add_gradient_f2d_kernel(long total, int K, const int *__restrict__ edges, const float *__restrict__ x,
-                                        const float *__restrict__ phi, double *__restrict__ z) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  long e = i / K;
-  int c = (int)(i % K);
-  int v0 = __ldg(edges + 2 * e), v1 = __ldg(edges + 2 * e + 1);
-  z[i] = (double)x[i] + ((double)__ldg(phi + (long)v1 * K + c) - (double)__ldg(phi + (long)v0 * K + c));
-}
-
-void add_gradient_f2d(int ne, int K, const int *edges, const float *x, const float *phi, double *z, cudaStream_t s) {
-  long total = (long)ne * K;
-  if (!total) return;
-  add_gradient_f2d_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(total, K, edges, x, phi, z);
-  EMG_LAUNCH_CHECK();
-}
-
-// z = x + G phi formed on the fly (FP64 from the FP32 AMS output and its
-// gradient potential), never stored: the FCG needs z only for its dot
-// products with the previous B-products and for the new direction
-__device__ __forceinline__ double zsplit_at(long i, int K, const int *__restrict__ edges,
-                                            const float *__restrict__ x, const float *__restrict__ phi) {
-  const long e = i / K;
-  const int c = (int)(i % K);
-  const int v0 = __ldg(edges + 2 * e), v1 = __ldg(edges + 2 * e + 1);
-  return (double)x[i] + ((double)__ldg(phi + (long)v1 * K + c) - (double)__ldg(phi + (long)v0 * K + c));
-}
-
-__global__ void __launch_bounds__(256) zsplit_dots_kernel(long total, int K, const int *__restrict__ edges,
-                                                          const float *__restrict__ x, const float *__restrict__ phi,
-                                                          int nprev, DevPtrs4 S, double *__restrict__ out) {
-  __shared__ double sh[4][256];
-  double acc[4] = {0, 0, 0, 0};
-  for (long i = blockIdx.x * 256L + threadIdx.x; i < total; i += (long)gridDim.x * 256) {
-    const double z = zsplit_at(i, K, edges, x, phi);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < nprev) acc[j] += z * S.p[j][i];
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) sh[j][threadIdx.x] = acc[j];
-  __syncthreads();
-  for (int st = 128; st >= K; st >>= 1) {
-    if ((int)threadIdx.x < st)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sh[j][threadIdx.x] += sh[j][threadIdx.x + st];
-    __syncthreads();
-  }
-  if ((int)threadIdx.x < K)
-    for (int j = 0; j < nprev; ++j) atomicAdd(out + j * K + threadIdx.x, sh[j][threadIdx.x]);
-}
-
-__global__ void zsplit_direction_kernel(long total, int K, const int *__restrict__ edges, const float *__restrict__ x,
-                                        const float *__restrict__ phi, int nprev, double *const *Pj,
-                                        const double *__restrict__ beta, double *__restrict__ p) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int c = (int)(i % K);
-  double v = zsplit_at(i, K, edges, x, phi);
-  for (int j = 0; j < nprev; ++j) v -= beta[j * K + c] * Pj[j][i];
-  p[i] = v;
-}
-
-void zsplit_dots(int n, int K, const int *edges, const float *x, const float *phi, int nprev, const DevPtrs4 &S,
-                 double *out, cudaStream_t s) {
-  const long total = (long)n * K;
-  if (nprev < 1 || nprev > 4) fail(EMG_ERR_ARG, "zsplit_dots: 1..4 previous directions");
-  zsplit_dots_kernel<<<red_grid(total), 256, 0, s>>>(total, K, edges, x, phi, nprev, S, out);
-  EMG_LAUNCH_CHECK();
-}
-
-void zsplit_direction(int n, int K, const int *edges, const float *x, const float *phi, int nprev,
-                      double *const *Pj, const double *beta, double *p, cudaStream_t s) {
-  const long total = (long)n * K;
-  zsplit_direction_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(total, K, edges, x, phi, nprev, Pj, beta,
-                                                                          p);
-  EMG_LAUNCH_CHECK();
-}
-
 template <typename T>
 void fill_zero(long count, T *a, cudaStream_t s) {
   if (count) EMG_CUDA(cudaMemsetAsync(a, 0, count * sizeof(T), s));
@@ -1172,11 +970,6 @@ void abs_bound2(int n, int K, const int *rp, const int *ci, const double *Cv, co
 
 // explicit instantiations
 #define EMG_INST(T)                                                                                              \
-  template void coldot<T>(int, int, const T *, const T *, double *, cudaStream_t);                              \
-  template void coldot3<T>(int, int, const T *, const T *, const T *, const T *, const T *, const T *, double *,  \
-                           cudaStream_t);                                                                        \
-  template void fcg_update<T>(int, int, const double *, const T *, const T *, T *, T *, double *, cudaStream_t, float *); \
-  template void fcg_direction<T>(int, int, const T *, int, T *const *, const double *, T *, cudaStream_t);       \
   template void jacobi0<T>(int, int, const T *, const T *, const T *, const double *, double, T *, T *,          \
                            cudaStream_t);                                                                        \
   template void fill_zero<T>(long, T *, cudaStream_t);                                                           \

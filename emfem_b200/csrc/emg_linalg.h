@@ -59,42 +59,14 @@ bool build_tiled(int n, const std::vector<int> &rp, const std::vector<int> &ci, 
 template <typename T>
 void spmm_tiled(int K, const SpmmArgs &a, const TiledPattern &tp, cudaStream_t s);
 
-// out[c] (+)= sum_i a[i*K+c] * b[i*K+c]   (FP64 accumulation); out must be zeroed
-template <typename T>
-void coldot(int n, int K, const T *a, const T *b, double *out, cudaStream_t s);
-// three dot products in one pass: out[0..K) = (a1,b1), out[K..2K) = (a2,b2), out[2K..3K) = (a3,b3)
-template <typename T>
-void coldot3(int n, int K, const T *a1, const T *b1, const T *a2, const T *b2, const T *a3, const T *b3,
-             double *out, cudaStream_t s);
-// x += alpha_c p ; r -= alpha_c s ; rn[c] += ||r_c||^2 ; r32 = (float) r when given
-template <typename T>
-void fcg_update(int n, int K, const double *alpha, const T *p, const T *sv, T *x, T *r, double *rn, cudaStream_t s,
-                float *r32 = nullptr);
-// p = z - sum_j beta[j*K+c] * P_j  (nprev directions, pointers in a device array)
-template <typename T>
-void fcg_direction(int n, int K, const T *z, int nprev, T *const *Pj, const double *beta, T *p, cudaStream_t st);
 // y (and d when given) = w * b / D  (first smoothing step from a zero guess)
 template <typename T>
 void jacobi0(int n, int K, const T *b, const T *l1c, const T *l1m, const double *omega, double w, T *y, T *d,
              cudaStream_t s);
 // precision conversion of block vectors
 void cvt_d2f(long count, const double *a, float *b, cudaStream_t s);
-void cvt_f2d(long count, const float *a, double *b, cudaStream_t s);
-// z = x + G phi in FP64 (edge e: phi[v1] - phi[v0]) for K columns
-void add_gradient_f2d(int ne, int K, const int *edges, const float *x, const float *phi, double *z, cudaStream_t s);
 template <typename T>
 void fill_zero(long count, T *a, cudaStream_t s);
-// FCG steps with z = x + G phi formed on the fly (FP32 AMS output x, FP32
-// gradient potential phi): out[j*K+c] += (z_c, S_j,c) for j < nprev (<= 4),
-// and p = z - sum_j beta[j*K+c] P_j
-struct DevPtrs4 {
-  const double *p[4];
-};
-void zsplit_dots(int n, int K, const int *edges, const float *x, const float *phi, int nprev, const DevPtrs4 &S,
-                 double *out, cudaStream_t s);
-void zsplit_direction(int n, int K, const int *edges, const float *x, const float *phi, int nprev,
-                      double *const *Pj, const double *beta, double *p, cudaStream_t s);
-
 // AMS transfers between edges and vertices for K columns.
 //   sp == 0: gradient G (row e: -1 at edges[e][0], +1 at edges[e][1])
 //   sp == 1..3: Pi_d, d = sp-1 (row e: 0.5 t_e[d] at both endpoints)

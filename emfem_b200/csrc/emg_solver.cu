@@ -44,24 +44,6 @@ __global__ void l1_rowsum_kernel(int n, const int *__restrict__ rp, const double
   out[i] = (T)s;
 }
 
-__global__ void fcg_beta_kernel(int K, int nprev, const double *__restrict__ dots, const double *__restrict__ eta,
-                                const int *__restrict__ active, double *__restrict__ beta) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= K * nprev) return;
-  int c = i % K;
-  double e = eta[i];
-  beta[i] = (active[c] && e != 0.0) ? dots[i] / e : 0.0;
-}
-
-__global__ void fcg_alpha_kernel(int K, const double *__restrict__ dots, double *__restrict__ eta_slot,
-                                 const int *__restrict__ active, double *__restrict__ alpha) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= K) return;
-  double ps = dots[c], pr = dots[K + c];
-  eta_slot[c] = ps;
-  alpha[c] = (active[c] && ps != 0.0) ? pr / ps : 0.0;
-}
-
 template <typename T>
 static void convert(const std::vector<double> &a, std::vector<T> &b) {
   b.resize(a.size());
@@ -866,7 +848,32 @@ void Ams<T>::launch_fused(int sp, cudaStream_t s) {
 // second is captured into a CUDA graph that every later call replays, so the
 // few hundred small launches of the nodal V-cycles cost one graph launch.
 template <typename T>
-void Ams<T>::apply(const T *b, T *x, cudaStream_t s) {
+void Ams<T>::signature(std::vector<uint64_t> &sig) const {
+  sig.push_back((uint64_t)this);
+  sig.push_back((uint64_t)graphs.epoch);
+  sig.push_back((uint64_t)ws_K);
+}
+
+template <typename T>
+T *Ams<T>::start_buffer(T *x) {
+  // out-of-place edge smoothing applications of a cycle decide where it
+  // starts, so that it ends in x
+  int zeros = 0;
+  for (char ch : cycle)
+    if (ch == '0') ++zeros;
+  const int sweeps = zeros * relax_times - (!cycle.empty() && cycle[0] == '0' ? 1 : 0);
+  return (sweeps & 1) ? ex2.p : x;
+}
+
+template <typename T>
+RestrictJ0<T> Ams<T>::edge_start(T *x) {
+  if (cycle.empty() || cycle[0] != '0') return RestrictJ0<T>{};
+  return RestrictJ0<T>{B.l1c.p, two ? B.l1m.p : nullptr, omega.p, cheb ? cheb_coef(cheb_degree).inv_theta : relax_w,
+                       start_buffer(x), cheb ? ed.p : nullptr};
+}
+
+template <typename T>
+void Ams<T>::apply(const T *b, T *x, cudaStream_t s, bool started) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   EMG_CUDA(cudaStreamIsCapturing(s, &cs));
   if (fused && cs == cudaStreamCaptureStatusNone) {
@@ -874,10 +881,10 @@ void Ams<T>::apply(const T *b, T *x, cudaStream_t s) {
     prepare_fused(s);
   }
   if (!use_graphs || cs != cudaStreamCaptureStatusNone || profiler().enabled) {
-    apply_eager(b, x, s);
+    apply_eager(b, x, s, started);
     return;
   }
-  auto key = std::make_pair((const void *)b, (void *)x);
+  auto key = std::make_pair((const void *)((const char *)b + (started ? 1 : 0)), (void *)x);
   auto it = graphs.exec.find(key);
   if (it != graphs.exec.end()) {
     EMG_CUDA(cudaGraphLaunch(it->second, s));
@@ -885,14 +892,14 @@ void Ams<T>::apply(const T *b, T *x, cudaStream_t s) {
     return;
   }
   if (graphs.seen[key]++ == 0) {
-    apply_eager(b, x, s);
+    apply_eager(b, x, s, started);
     return;
   }
   cudaGraph_t g;
   const long l0 = launch_count();
   EMG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
-    apply_eager(b, x, s);
+    apply_eager(b, x, s, started);
   } catch (...) {
     cudaStreamEndCapture(s, &g);
     if (g) cudaGraphDestroy(g);
@@ -919,22 +926,16 @@ void Ams<T>::grad_vcycle(const T *b, T *x, cudaStream_t s) {
 }
 
 template <typename T>
-void Ams<T>::apply_eager(const T *b, T *x, cudaStream_t s) {
-  // count out-of-place edge smoothing applications to choose the start buffer
-  int zeros = 0;
-  for (char ch : cycle)
-    if (ch == '0') ++zeros;
-  const bool starts_with_smoother = !cycle.empty() && cycle[0] == '0';
-  const int sweeps = zeros * relax_times - (starts_with_smoother ? 1 : 0);
-  T *cur = (sweeps & 1) ? ex2.p : x;
-  T *oth = (sweeps & 1) ? x : ex2.p;
+void Ams<T>::apply_eager(const T *b, T *x, cudaStream_t s, bool started_edge) {
+  T *cur = start_buffer(x);
+  T *oth = cur == x ? ex2.p : x;
   const char *bin = sizeof(T) == 4 ? "spmm_edge_fp32" : "spmm_edge_fp64";
   bool zero = true;
   for (size_t ci = 0; ci < cycle.size(); ++ci) {
     const char ch = cycle[ci];
     if (ch == '0') {
       for (int it = 0; it < relax_times; ++it) {
-        T *res = smooth(nullptr, nnzB, ne, cur, oth, b, er.p, ed.p, ed2.p, zero, bin, s);
+        T *res = smooth(nullptr, nnzB, ne, cur, oth, b, er.p, ed.p, ed2.p, zero, bin, s, zero && started_edge);
         if (res != cur) std::swap(cur, oth);
         zero = false;
       }
@@ -1007,188 +1008,18 @@ size_t Ams<T>::device_bytes() const {
   return b;
 }
 
-// ---------------------------------------------------------------------------
-// batched FCG
-// ---------------------------------------------------------------------------
-template <typename T>
-int Fcg<T>::solve(Ams<T> &ams, const T *b, T *x, double rtol, int maxit, cudaStream_t s) {
-  return solve_with(
-      ams.ne, ams.K, [&](const T *r_, T *z_) { ams.apply(r_, z_, s); },
-      [&](const T *p_, T *s_) { ams.spmm_B(SPMM_AX, p_, nullptr, s_, s); }, b, x, rtol, maxit, s);
-}
-
-// device-side column bookkeeping of the batched FCG: no host round trip per
-// iteration
-__global__ void fcg_init_kernel(int K, const double *__restrict__ bn, int *__restrict__ act, int *__restrict__ its,
-                                int *__restrict__ status) {
-  const int c = threadIdx.x;
-  if (c < K) {
-    act[c] = bn[c] > 0.0;
-    its[c] = 0;
-  }
-  if (c == 0) status[0] = status[1] = 0;
-}
-
-// after an update: count the iteration of every active column, retire the
-// converged ones (||r_c||^2 <= rtol^2 ||b_c||^2), flag NaN/Inf; status[0] =
-// active columns left, status[1] = 1 + the first non-finite column (0: none)
-__global__ void fcg_status_kernel(int K, const double *__restrict__ rn, const double *__restrict__ bn, double rtol2,
-                                  int *__restrict__ act, int *__restrict__ its, int *__restrict__ status) {
-  const int c = threadIdx.x;
-  int a = 0;
-  if (c < K && act[c]) {
-    its[c]++;
-    const double v = rn[c];
-    if (!isfinite(v)) {
-      atomicCAS(status + 1, 0, c + 1);
-      act[c] = 0;
-    } else if (v <= rtol2 * bn[c]) {
-      act[c] = 0;
-    } else {
-      a = 1;
-    }
-  }
-  const int n = __syncthreads_count(a);
-  if (c == 0) status[0] = n;
-}
-
-template <typename T>
-int Fcg<T>::solve_with(int n, int Kc, const std::function<void(const T *, T *)> &pc,
-                       const std::function<void(const T *, T *)> &opB, const T *b, T *x, double rtol, int maxit,
-                       cudaStream_t s, float *r32, const ZSplit *zs) {
-  K = Kc;
-  if (zs && (sizeof(T) != 8 || mmax > 4)) fail(EMG_ERR_STATE, "split z needs FP64 recurrences and at most 4 directions");
-  const size_t N = (size_t)n * K;
-  if (mmax < 1) mmax = 1;
-  if (K > 1024) fail(EMG_ERR_ARG, "batched FCG supports at most 1024 columns");
-  r.alloc(N);
-  z.alloc(N);
-  bool new_ring = false;
-  if ((int)P.size() != mmax || P.empty() || P[0].n != N) {
-    P.clear();
-    S.clear();
-    P.resize(mmax);
-    S.resize(mmax);
-    for (int j = 0; j < mmax; ++j) {
-      P[j].alloc(N);
-      S[j].alloc(N);
-    }
-    new_ring = true;
-  }
-  dots.alloc((size_t)(mmax + 3) * K);
-  eta.alloc((size_t)mmax * K);
-  eord.alloc((size_t)mmax * K);
-  alpha.alloc(K);
-  beta.alloc((size_t)mmax * K);
-  rn.alloc(K);
-  bn.alloc(K);
-  act.alloc(K);
-  itsd.alloc(K);
-  status.alloc(2);
-  if (!h_status.p) EMG_CUDA(cudaMallocHost((void **)&h_status.p, 2 * sizeof(int)));
-  // ring orderings: for (head, nprev) the previous directions oldest first
-  if (new_ring || ptab_mmax != mmax || ptrs.n != (size_t)mmax * (mmax + 1) * mmax) {
-    std::vector<T *> tab((size_t)mmax * (mmax + 1) * mmax, nullptr);
-    for (int h = 0; h < mmax; ++h)
-      for (int np = 1; np <= mmax; ++np)
-        for (int j = 0; j < np; ++j) tab[((size_t)h * (mmax + 1) + np) * mmax + j] = P[(h - np + j + mmax) % mmax].p;
-    ptrs.upload(tab, s);
-    EMG_CUDA(cudaStreamSynchronize(s));
-    ptab_mmax = mmax;
-  }
-  its.assign(K, 0);
-  fill_zero<T>((long)N, x, s);
-  EMG_CUDA(cudaMemcpyAsync(r.p, b, sizeof(T) * N, cudaMemcpyDeviceToDevice, s));
-  if (r32) {
-    if (sizeof(T) != 8) fail(EMG_ERR_STATE, "FP32 residual copy needs FP64 recurrences");
-    cvt_d2f((long)N, reinterpret_cast<const double *>(b), r32, s);
-  }
-  bn.zero(s);
-  coldot<T>(n, K, b, b, bn.p, s);
-  fcg_init_kernel<<<1, 1024, 0, s>>>(K, bn.p, act.p, itsd.p, status.p);
-  EMG_LAUNCH_CHECK();
-  const int every = std::max(1, check_every);
-  int nprev = 0, head = 0, it = 0;
-  for (it = 0; it < maxit; ++it) {
-    pc(r.p, z.p);
-    if (zs) {
-      // z = x + G phi only inside these two passes
-      if (nprev > 0) {
-        EMG_CUDA(cudaMemsetAsync(dots.p, 0, sizeof(double) * nprev * K, s));
-        DevPtrs4 Sj{{nullptr, nullptr, nullptr, nullptr}};
-        for (int j = 0; j < nprev; ++j) {
-          const int sl = (head - nprev + j + mmax) % mmax;
-          Sj.p[j] = reinterpret_cast<const double *>(S[sl].p);
-          EMG_CUDA(cudaMemcpyAsync(eord.p + (size_t)j * K, eta.p + (size_t)sl * K, sizeof(double) * K,
-                                   cudaMemcpyDeviceToDevice, s));
-        }
-        zsplit_dots(n, K, zs->edges, zs->x, zs->phi, nprev, Sj, dots.p, s);
-        fcg_beta_kernel<<<(nprev * K + 127) / 128, 128, 0, s>>>(K, nprev, dots.p, eord.p, act.p, beta.p);
-        EMG_LAUNCH_CHECK();
-      }
-      zsplit_direction(n, K, zs->edges, zs->x, zs->phi, nprev,
-                       reinterpret_cast<double *const *>(ptrs.p + ((size_t)head * (mmax + 1) + nprev) * mmax),
-                       beta.p, reinterpret_cast<double *>(P[head].p), s);
-    } else if (nprev > 0) {
-      EMG_CUDA(cudaMemsetAsync(dots.p, 0, sizeof(double) * nprev * K, s));
-      for (int j = 0; j < nprev; ++j) {
-        const int sl = (head - nprev + j + mmax) % mmax;
-        coldot<T>(n, K, z.p, S[sl].p, dots.p + (size_t)j * K, s);
-        // eta of the ring slots in the same order
-        EMG_CUDA(cudaMemcpyAsync(eord.p + (size_t)j * K, eta.p + (size_t)sl * K, sizeof(double) * K,
-                                 cudaMemcpyDeviceToDevice, s));
-      }
-      fcg_beta_kernel<<<(nprev * K + 127) / 128, 128, 0, s>>>(K, nprev, dots.p, eord.p, act.p, beta.p);
-      EMG_LAUNCH_CHECK();
-      fcg_direction<T>(n, K, z.p, nprev, ptrs.p + ((size_t)head * (mmax + 1) + nprev) * mmax, beta.p, P[head].p,
-                       s);
-    } else {
-      EMG_CUDA(cudaMemcpyAsync(P[head].p, z.p, sizeof(T) * N, cudaMemcpyDeviceToDevice, s));
-    }
-    T *p = P[head].p;
-    T *sv = S[head].p;
-    opB(p, sv);
-    EMG_CUDA(cudaMemsetAsync(dots.p, 0, sizeof(double) * 2 * K, s));
-    coldot3<T>(n, K, p, sv, p, r.p, nullptr, nullptr, dots.p, s);
-    fcg_alpha_kernel<<<(K + 63) / 64, 64, 0, s>>>(K, dots.p, eta.p + (size_t)head * K, act.p, alpha.p);
-    EMG_LAUNCH_CHECK();
-    rn.zero(s);
-    fcg_update<T>(n, K, alpha.p, p, sv, x, r.p, rn.p, s, r32);
-    fcg_status_kernel<<<1, 1024, 0, s>>>(K, rn.p, bn.p, rtol * rtol, act.p, itsd.p, status.p);
-    EMG_LAUNCH_CHECK();
-    head = (head + 1) % mmax;
-    nprev = std::min(nprev + 1, mmax);
-    // the host looks at the column status only every `every` iterations (and
-    // at the cap); columns that converged in between stay frozen (alpha = beta
-    // = 0 keeps x and r)
-    if (verbose || (it + 1) % every == 0 || it + 1 == maxit) {
-      EMG_CUDA(cudaMemcpyAsync(h_status.p, status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-      EMG_CUDA(cudaStreamSynchronize(s));
-      if (verbose) {
-        std::vector<double> ha(K), hrn(K), hbn(K);
-        alpha.download(ha.data(), K, s);
-        rn.download(hrn.data(), K, s);
-        bn.download(hbn.data(), K, s);
-        EMG_CUDA(cudaStreamSynchronize(s));
-        fprintf(stderr, "fcg it %d:", it);
-        for (int c = 0; c < K; ++c)
-          fprintf(stderr, " [%d a=%.3e r=%.3e]", c, ha[c], std::sqrt(hrn[c] / std::max(hbn[c], 1e-300)));
-        fprintf(stderr, "\n");
-      }
-      if (h_status.p[1]) fail(EMG_DIVERGED_NANORINF, "inner FCG: NaN or Inf in the residual of column %d",
-                              h_status.p[1] - 1);
-      if (h_status.p[0] == 0) {
-        ++it;
-        break;
-      }
-    }
-  }
-  itsd.download(its.data(), K, s);
-  EMG_CUDA(cudaStreamSynchronize(s));
-  long tot = 0;
-  for (int c = 0; c < K; ++c) tot += its[c];
-  total_its += tot;
-  return it;
+int fcg_solve(Fcg &fcg, Ams<double> &ams, const double *b, double *x, double rtol, int maxit, cudaStream_t s) {
+  std::vector<uint64_t> sig;
+  const KernelProfiler &pf = profiler();
+  if (ams.use_graphs && !ams.fused && !pf.enabled && !pf.phases) ams.signature(sig);
+  fcg.z.alloc((size_t)ams.ne * ams.K);
+  FcgFeed feed;
+  feed.jd = ams.edge_start(fcg.z.p);
+  const bool started = feed.jd.y != nullptr;
+  return fcg.solve(
+      ams.ne, ams.K, [&](const double *r_, double *z_) { ams.apply(r_, z_, s, started); },
+      [&](const double *p_, double *s_) { ams.spmm_B(SPMM_AX, p_, nullptr, s_, s); }, b, x, rtol, maxit, s, feed,
+      nullptr, sig);
 }
 
 // ---------------------------------------------------------------------------
@@ -1608,7 +1439,5 @@ template void ams_setup<float>(Context &, Ams<float> &, bool, double, double);
 template void ams_setup<double>(Context &, Ams<double> &, bool, double, double);
 template struct Ams<float>;
 template struct Ams<double>;
-template struct Fcg<float>;
-template struct Fcg<double>;
 
 }  // namespace emg

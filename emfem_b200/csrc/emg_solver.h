@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "emg_amg.h"
+#include "emg_fcg.h"
 #include "emg_internal.h"
 #include "emg_linalg.h"
 
@@ -45,28 +46,6 @@ struct GraphCache {
     exec.clear();
     seen.clear();
     kernels.clear();
-  }
-};
-
-// one pinned host word (move-only)
-struct PinnedWord {
-  int *p = nullptr;
-  PinnedWord() = default;
-  PinnedWord(const PinnedWord &) = delete;
-  PinnedWord &operator=(const PinnedWord &) = delete;
-  PinnedWord(PinnedWord &&o) noexcept : p(o.p) { o.p = nullptr; }
-  PinnedWord &operator=(PinnedWord &&o) noexcept {
-    if (this != &o) {
-      release();
-      p = o.p;
-      o.p = nullptr;
-    }
-    return *this;
-  }
-  ~PinnedWord() { release(); }
-  void release() {
-    if (p) cudaFreeHost(p);
-    p = nullptr;
   }
 };
 
@@ -156,8 +135,16 @@ struct Ams {
   std::vector<DBuf<T>> wb[NSUB], wx[NSUB], wr[NSUB], wx2[NSUB], wd[NSUB], wd2[NSUB];
 
   void set_columns(const std::vector<double> &col_omega, cudaStream_t s);
-  void apply(const T *b, T *x, cudaStream_t s);
-  void apply_eager(const T *b, T *x, cudaStream_t s);
+  // started: the caller has taken the first zero-guess edge smoothing step
+  // into the buffers of edge_start(x)
+  void apply(const T *b, T *x, cudaStream_t s, bool started = false);
+  void apply_eager(const T *b, T *x, cudaStream_t s, bool started = false);
+  // where an application into x starts (y null when its cycle does not begin
+  // with edge smoothing)
+  RestrictJ0<T> edge_start(T *x);
+  // address of its state and version of the addresses behind it
+  void signature(std::vector<uint64_t> &sig) const;
+  T *start_buffer(T *x);
   const T *gphi() const { return wx[0][0].p; }  // gradient potential (split form)
   // one V-cycle of the gradient space's nodal hierarchy on K vertex columns
   // (b, x: nv x K, device); the divergence correction's preconditioner
@@ -203,43 +190,13 @@ struct Ams {
 template <typename T>
 void ams_setup(Context &c, Ams<T> &ams, bool per_frequency, double w, double w_ref);
 
+// two FCG solves on the real and imaginary columns (pc_apply_b): B x = b with
+// the FP64 AMS
+int fcg_solve(Fcg &fcg, Ams<double> &ams, const double *b, double *x, double rtol, int maxit, cudaStream_t s);
+
 // tests: rows, nonzeros and absolute sums per level of a nodal hierarchy
 // built on the device (gpu) or on the host
 void amg_levels_report(Context &c, int sp, bool gpu, double w_ref, std::vector<double> &out);
-
-// batched FCG on B(w_c) with AMS, K real columns; returns per-column iteration
-// counts; x starts at zero.  Columns converge independently to
-// ||r_c|| <= rtol ||b_c|| (unpreconditioned norm, src/em_la.cc:120).
-template <typename T>
-struct Fcg {
-  int K = 0;
-  int mmax = 1;
-  DBuf<T> r, z, p;
-  std::vector<DBuf<T>> P, S;  // previous directions and B-products (ring)
-  DBuf<double> dots, eta, eord, alpha, beta, rn, bn;
-  DBuf<T *> ptrs;          // ring orderings of the previous directions, per (head, nprev)
-  int ptab_mmax = 0;
-  DBuf<int> act, itsd, status;  // per-column activity and iteration counts; active count, NaN flag
-  PinnedWord h_status;          // two words (see fcg_status_kernel)
-  std::vector<int> its;
-  long total_its = 0;
-  int verbose = 0;
-  int check_every = 1;     // iterations between host looks at the column status
-  int solve(Ams<T> &ams, const T *b, T *x, double rtol, int maxit, cudaStream_t s);
-  // generic form: pc(r, z) applies the preconditioner, opB(p, s) the operator;
-  // n rows, K columns
-  // r32: when given, kept equal to (float) r for an FP32 preconditioner
-  // zs: the preconditioner leaves z split as x + G phi in FP32 (zs->x, zs->phi
-  // over the edges zs->edges) instead of writing z; the dot products and the
-  // direction then form z on the fly
-  struct ZSplit {
-    const int *edges;
-    const float *x, *phi;
-  };
-  int solve_with(int n, int Kc, const std::function<void(const T *, T *)> &pc,
-                 const std::function<void(const T *, T *)> &opB, const T *b, T *x, double rtol, int maxit,
-                 cudaStream_t s, float *r32 = nullptr, const ZSplit *zs = nullptr);
-};
 
 struct SolveStats {
   int outer_its = 0;
