@@ -912,9 +912,7 @@ int emg_matshell_mult_a(emg_context *c, const double *x, double *y) {
   Workspace &w = *c->ws;
   w.vec_a.upload(xi, c->stream);
   w.vec_b.alloc((size_t)n * 2);
-  w.omega_k.upload(&c->omega, 1, c->stream);
-  spmm_complex(n, 1, c->rp.p, c->ci.p, c->Cv.p, c->Msv.p, w.omega_k.p, w.vec_a.p, nullptr, w.vec_b.p, false, true,
-               c->stream);
+  spmm_complex_host(n, 1, c->rp.p, c->ci.p, c->Cv.p, c->Msv.p, &c->omega, w.vec_a.p, w.vec_b.p, true, c->stream);
   std::vector<double> yo((size_t)n * 2);
   w.vec_b.download(yo.data(), yo.size(), c->stream);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1864,9 +1862,7 @@ int emg_spmv_complex_dev(emg_context *c, int k, const double *omegas, const doub
   need(c && omegas && x_dev && y_dev, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "operator not assembled");
   use_device(*c);
-  c->ws->omega_k.upload(omegas, k, c->stream);
-  spmm_complex(c->ne, k, c->rp.p, c->ci.p, c->Cv.p, c->Msv.p, c->ws->omega_k.p, x_dev, nullptr, y_dev, false,
-               conj_out != 0, c->stream);
+  spmm_complex_host(c->ne, k, c->rp.p, c->ci.p, c->Cv.p, c->Msv.p, omegas, x_dev, y_dev, conj_out != 0, c->stream);
   EMG_API_END
 }
 

@@ -710,74 +710,130 @@ void coarse_apply(int nc, int K, const double *inv, const int *col_slot, const T
 // ---------------------------------------------------------------------------
 // complex FP64 kernels of the outer FGMRES
 // ---------------------------------------------------------------------------
-template <int K, int NL>
-__global__ void __launch_bounds__(256) spmm_complex_kernel(int n, const int *__restrict__ rp,
+// column frequencies as a kernel argument
+struct Omegas {
+  double w[32];
+};
+
+// y = A(w_c) x or b - A(w_c) x: CL = K / V lanes of V columns per row, NL lanes
+// splitting its nonzeros, U nonzeros per lane and round; the index and value
+// loads of a round go out before its gathers.  The data pipe of L1 is the
+// busiest unit (66 % at K = 16, 1.81M rows; L2 21 %, DRAM 26 %): a warp-wide
+// load that touches several rows costs a pass per row, so few lanes per row
+// with two columns each share the three matrix loads of a nonzero best.
+// Measured: 806 -> 685 us at K = 16, 1.81M rows (V = 2, 3 blocks per SM; V = 1
+// 842, V = 4 789, two rows per warp with split nonzeros 1111).
+template <int K, int V, int NL, int U, int MINB>
+__global__ void __launch_bounds__(256, MINB) spmm_complex_kernel(int n, const int *__restrict__ rp,
                                                            const int *__restrict__ ci, const double *__restrict__ Cv,
                                                            const double *__restrict__ Mv,
                                                            const double *__restrict__ omega,
+                                                           const __grid_constant__ Omegas by_value,
                                                            const double2 *__restrict__ x,
                                                            const double2 *__restrict__ b, double2 *__restrict__ y,
                                                            bool residual, bool conj_out) {
-  constexpr int G = K * NL;
+  constexpr int CL = K / V, G = CL * NL;
   const int lane = threadIdx.x & 31;
-  const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int row = gwarp * (32 / G) + lane / G;
+  const int row = (int)((blockIdx.x * 256L + threadIdx.x) / G);
   const int sub = lane % G;
-  const int c = sub % K, sl = sub / K;
-  const double w = __ldg(omega + c);
-  double ar = 0, ai = 0;
+  const int cl = sub % CL, sl = sub / CL;
+  double w[V], ar[V], ai[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    w[i] = omega ? __ldg(omega + cl + i * CL) : by_value.w[cl + i * CL];
+    ar[i] = ai[i] = 0;
+  }
   const bool valid = row < n;
   if (valid) {
-    const int kb = __ldg(rp + row), ke = __ldg(rp + row + 1);
-    for (int k = kb + sl; k < ke; k += NL) {
-      const int j = __ldg(ci + k);
-      const double a = __ldg(Cv + k), m = w * __ldg(Mv + k);
-      const double2 xv = __ldg(x + (long)j * K + c);
-      ar = fma(a, xv.x, fma(-m, xv.y, ar));
-      ai = fma(a, xv.y, fma(m, xv.x, ai));
+    const int ke = __ldg(rp + row + 1);
+    for (int k0 = __ldg(rp + row) + sl; k0 < ke; k0 += NL * U) {
+      int j[U];
+      double a[U], m[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + u * NL;
+        const bool ok = k < ke;
+        j[u] = ok ? __ldg(ci + k) : -1;
+        a[u] = ok ? __ldg(Cv + k) : 0.0;
+        m[u] = ok ? __ldg(Mv + k) : 0.0;
+      }
+      double2 xv[U][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+          xv[u][i] = j[u] >= 0 ? __ldg(x + (long)j[u] * K + cl + i * CL) : make_double2(0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const double mw = w[i] * m[u];
+          ar[i] = fma(a[u], xv[u][i].x, fma(-mw, xv[u][i].y, ar[i]));
+          ai[i] = fma(a[u], xv[u][i].y, fma(mw, xv[u][i].x, ai[i]));
+        }
     }
   }
 #pragma unroll
-  for (int off = K; off < G; off <<= 1) {
-    ar += __shfl_xor_sync(0xffffffffu, ar, off);
-    ai += __shfl_xor_sync(0xffffffffu, ai, off);
-  }
+  for (int off = CL; off < G; off <<= 1)
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      ar[i] += __shfl_xor_sync(0xffffffffu, ar[i], off);
+      ai[i] += __shfl_xor_sync(0xffffffffu, ai[i], off);
+    }
   if (!valid || sl != 0) return;
-  if (conj_out) ai = -ai;
-  const long o = (long)row * K + c;
-  if (residual) {
-    double2 bv = __ldg(b + o);
-    y[o] = make_double2(bv.x - ar, bv.y - ai);
-  } else {
-    y[o] = make_double2(ar, ai);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    if (conj_out) ai[i] = -ai[i];
+    const long o = (long)row * K + cl + i * CL;
+    if (residual) {
+      const double2 bv = __ldg(b + o);
+      ar[i] = bv.x - ar[i];
+      ai[i] = bv.y - ai[i];
+    }
+    y[o] = make_double2(ar[i], ai[i]);
   }
 }
 
-template <int K>
+template <int K, int V, int NL, int U, int MINB>
 static void spmm_complex_k(int n, const int *rp, const int *ci, const double *Cv, const double *Mv,
-                           const double *omega, const double *x, const double *b, double *y, bool residual,
-                           bool conj_out, cudaStream_t s) {
-  constexpr int NL = (32 / K) >= 8 ? 8 : (32 / K);
-  constexpr int RPW = 32 / (K * NL);
-  long warps = ((long)n + RPW - 1) / RPW;
-  unsigned grid = (unsigned)((warps * 32 + 255) / 256);
-  spmm_complex_kernel<K, NL><<<grid, 256, 0, s>>>(n, rp, ci, Cv, Mv, omega, (const double2 *)x, (const double2 *)b,
-                                                  (double2 *)y, residual, conj_out);
+                           const double *omega, const Omegas &om, const double *x, const double *b, double *y,
+                           bool residual, bool conj_out, cudaStream_t s) {
+  const unsigned grid = (unsigned)(((long)n * (K / V * NL) + 255) / 256);
+  spmm_complex_kernel<K, V, NL, U, MINB><<<grid, 256, 0, s>>>(n, rp, ci, Cv, Mv, omega, om, (const double2 *)x,
+                                                              (const double2 *)b, (double2 *)y, residual, conj_out);
   EMG_LAUNCH_CHECK();
+}
+
+static void spmm_complex_any(int n, int K, const int *rp, const int *ci, const double *Cv, const double *Mv,
+                             const double *omega, const Omegas &om, const double *x, const double *b, double *y,
+                             bool residual, bool conj_out, cudaStream_t s) {
+  if (n <= 0) return;
+  auto run = [&](auto f) { f(n, rp, ci, Cv, Mv, omega, om, x, b, y, residual, conj_out, s); };
+  // narrow blocks split a row over lanes (16 nonzeros in one round); from 8
+  // columns on a row's lanes are its columns
+  switch (K) {
+  case 1: return run(&spmm_complex_k<1, 1, 4, 4, 1>);
+  case 2: return run(&spmm_complex_k<2, 1, 2, 4, 4>);
+  case 4: return run(&spmm_complex_k<4, 1, 2, 4, 4>);
+  case 8: return run(&spmm_complex_k<8, 1, 1, 4, 4>);
+  case 16: return run(&spmm_complex_k<16, 2, 1, 4, 3>);
+  case 32: return run(&spmm_complex_k<32, 2, 1, 4, 3>);
+  }
+  fail(EMG_ERR_ARG, "unsupported complex block width %d", K);
 }
 
 void spmm_complex(int n, int K, const int *rp, const int *ci, const double *Cv, const double *Mv,
                   const double *omega, const double *x, const double *b, double *y, bool residual, bool conj_out,
                   cudaStream_t s) {
-  switch (K) {
-  case 1: return spmm_complex_k<1>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  case 2: return spmm_complex_k<2>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  case 4: return spmm_complex_k<4>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  case 8: return spmm_complex_k<8>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  case 16: return spmm_complex_k<16>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  case 32: return spmm_complex_k<32>(n, rp, ci, Cv, Mv, omega, x, b, y, residual, conj_out, s);
-  }
-  fail(EMG_ERR_ARG, "unsupported complex block width %d", K);
+  spmm_complex_any(n, K, rp, ci, Cv, Mv, omega, Omegas{}, x, b, y, residual, conj_out, s);
+}
+
+void spmm_complex_host(int n, int K, const int *rp, const int *ci, const double *Cv, const double *Mv,
+                       const double *omega_host, const double *x, double *y, bool conj_out, cudaStream_t s) {
+  Omegas om{};
+  if (K < 1 || K > 32) fail(EMG_ERR_ARG, "unsupported complex block width %d", K);
+  std::copy(omega_host, omega_host + K, om.w);
+  spmm_complex_any(n, K, rp, ci, Cv, Mv, nullptr, om, x, nullptr, y, false, conj_out, s);
 }
 
 constexpr int MAXJ = 32;

@@ -125,7 +125,7 @@ struct FusedOp {
 // `row`) and stores the results.
 template <typename T, int V>
 struct EpiIn {
-  T b[V], x[V], r[V], y[V];
+  T b[V], x[V], y[V];  // b: a.b, or a.r of SPMM_CHEB2 (one array: fewer registers, fewer spills)
   T dc, dm;
 };
 
@@ -152,7 +152,7 @@ __device__ __forceinline__ void epi_load(const SpmmArgs &a, int row, int cb, Epi
   if (mode == SPMM_RES || mode == SPMM_JAC || mode == SPMM_CHEB1 || mode == SPMM_CHEBK || mode == SPMM_RESJ0)
     ldv<T, V>(static_cast<const T *>(a.b) + o, e.b);
   if (mode == SPMM_JAC || cheb) ldv<T, V>(x + o, e.x);
-  if (mode == SPMM_CHEB2) ldv<T, V>(static_cast<const T *>(a.r) + o, e.r);
+  if (mode == SPMM_CHEB2) ldv<T, V>(static_cast<const T *>(a.r) + o, e.b);
   if (mode == SPMM_ADD || mode == SPMM_CHEB2 || mode == SPMM_CHEBK) ldv<T, V>(y + o, e.y);
 }
 
@@ -225,7 +225,7 @@ __device__ __forceinline__ void epi_store(const SpmmArgs &a, int row, int cb, co
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       T dg = two ? e.dc + w[i] * e.dm : e.dc;
-      out[i] = e.y[i] + (T)a.c1 * e.x[i] + (T)a.c2 * (e.r[i] - acc[i]) / dg;
+      out[i] = e.y[i] + (T)a.c1 * e.x[i] + (T)a.c2 * (e.b[i] - acc[i]) / dg;
     }
   }
   stv<T, V>(y + o, out);

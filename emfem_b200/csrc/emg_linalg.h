@@ -108,6 +108,10 @@ void vcycle_fused(int K, const FusedOp *ops, int nops, unsigned *bar, int *err, 
 void spmm_complex(int n, int K, const int *rp, const int *ci, const double *Cv, const double *Mv,
                   const double *omega, const double *x, const double *b, double *y, bool residual, bool conj_out,
                   cudaStream_t s);
+// y = A(w_c) x with the column frequencies in host memory (they travel with
+// the launch instead of in a copy of their own)
+void spmm_complex_host(int n, int K, const int *rp, const int *ci, const double *Cv, const double *Mv,
+                       const double *omega_host, const double *x, double *y, bool conj_out, cudaStream_t s);
 // h[j*K+c] = sum_i conj(V_j[i,c]) w[i,c]  for j < J (complex), V_j = V + j*stride
 void cmultidot(int n, int K, int J, const double *V, long stride, const double *w, double *h, double *partial,
                int partial_blocks, cudaStream_t s);
