@@ -1,11 +1,10 @@
-// Element-matrix generation and scatter into the precomputed CSR pattern.
+// Element-matrix generation and row-wise assembly into the CSR pattern.
 //
 // Replaces the tet loop of assemble_matrix (src/em_fwd.cc:343-392): one
-// thread computes the closed-form Whitney element matrices of one tet (the
-// 4-point rule of em_fe.cc:82-128 is exact for these integrands, so the
-// closed form equals the reference up to rounding), stages them in shared
-// memory, and the warp then scatters its 32 tets' 36+36 entries with
-// coalesced reads of the tet->slot map and FP64 atomic adds.
+// thread per matrix row evaluates the edge's row of the closed-form Whitney
+// element matrices of the tets around it (the 4-point rule of em_fe.cc:82-128
+// is exact for these integrands, so the closed form equals the reference up to
+// rounding) and sums them in a shared tile of the row's slots.
 //
 // C is omega-independent and the mass part is stored without omega (Ms);
 // the reference's M is omega * Ms (src/em_fwd.cc:336,365).
@@ -114,6 +113,9 @@ void build_sparsity(Context &c) {
   }
   c.rp.upload(c.h_rp, c.stream);
   c.ci.upload(c.h_ci, c.stream);
+  c.einc_rp.upload(e2t_rp, c.stream);
+  c.einc.upload(e2t, c.stream);
+  EMG_CUDA(cudaStreamSynchronize(c.stream));  // the incidence lists go out of scope
 }
 
 // vertex adjacency (pattern of G^T B G and Pi^T B Pi) and vertex->edge incidence
@@ -168,14 +170,67 @@ __device__ __forceinline__ int find_col(const int *__restrict__ ci, int b, int e
   return lo;
 }
 
-// slot[t*36 + k*6 + l] = CSR slot of (cedge[t][k], cedge[t][l])
-__global__ void slot_map_kernel(int nt, const int *__restrict__ cedge, const int *__restrict__ rp,
-                                const int *__restrict__ ci, int *__restrict__ slot) {
-  long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long)nt * 36) return;
-  int t = (int)(idx / 36), ent = (int)(idx % 36);
-  int row = __ldg(cedge + 6 * (long)t + ent / 6), col = __ldg(cedge + 6 * (long)t + ent % 6);
-  slot[idx] = find_col(ci, __ldg(rp + row), __ldg(rp + row + 1), col);
+// Record of an (edge, tet) incidence for assemble_edge_kernel.  The tet's
+// vertices are taken in the order (a, b, c, d): a < b the edge's end points,
+// c < d the other two; its edges in the order ab, ac, ad, bc, bd, cd.
+//   einc[j]: the tet, with its canonical edge index k in bits 28..30
+//   erec[j]: 9 bits per edge: its position in the row (511: search for it),
+//            bits 54..57: whether c < a, d < a, c < b, d < b (the edge then
+//            runs against its global orientation), bits 58..63: whether each
+//            edge is on the boundary
+constexpr int kTetBits = 28;
+constexpr unsigned kSearch = 511;
+
+// positions (in the sorted tet) of the vertices a, b, c, d for edge k
+__host__ __device__ constexpr int kOther(int k, int which) {
+  return which == 0 ? (kEdgeP(k) == 0 ? (kEdgeQ(k) == 1 ? 2 : 1) : 0)
+                    : (kEdgeQ(k) == 3 ? (kEdgeP(k) == 2 ? 1 : 2) : 3);
+}
+// canonical edge joining sorted positions i < j
+__host__ __device__ constexpr int kEdgeOf(int i, int j) { return i == 0 ? j - 1 : (i == 1 ? j + 1 : 5); }
+
+__global__ void edge_records_kernel(int ne, const int *__restrict__ inc_rp, int *__restrict__ inc,
+                                    const int *__restrict__ cedge, const unsigned char *__restrict__ ebdr,
+                                    const int *__restrict__ rp, const int *__restrict__ ci,
+                                    unsigned long long *__restrict__ rec) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  const int kb = __ldg(rp + e), ke = __ldg(rp + e + 1);
+  for (int j = __ldg(inc_rp + e); j < __ldg(inc_rp + e + 1); ++j) {
+    const int t = inc[j];
+    int ge[6], k = 0;
+    for (int l = 0; l < 6; ++l) {
+      ge[l] = __ldg(cedge + 6 * (long)t + l);
+      if (ge[l] == e) k = l;
+    }
+    const int v[4] = {kEdgeP(k), kEdgeQ(k), kOther(k, 0), kOther(k, 1)};
+    unsigned long long r = 0;
+    int q = 0;
+    for (int x = 0; x < 4; ++x)
+      for (int y = x + 1; y < 4; ++y, ++q) {
+        const int lo = min(v[x], v[y]), hi = max(v[x], v[y]), g = ge[kEdgeOf(lo, hi)];
+        const int pos = find_col(ci, kb, ke, g) - kb;
+        r |= (unsigned long long)(pos < (int)kSearch ? (unsigned)pos : kSearch) << (9 * q);
+        if (__ldg(ebdr + g)) r |= 1ull << (58 + q);
+      }
+    if (v[2] < v[0]) r |= 1ull << 54;
+    if (v[3] < v[0]) r |= 1ull << 55;
+    if (v[2] < v[1]) r |= 1ull << 56;
+    if (v[3] < v[1]) r |= 1ull << 57;
+    rec[j] = r;
+    inc[j] = t | (k << kTetBits);
+  }
+}
+
+// whether a tet touches a boundary edge (ctx->bdr_cells, src/em_fwd.cc:377-388)
+__global__ void bdr_cell_kernel(int nt, const int *__restrict__ cedge, const unsigned char *__restrict__ ebdr,
+                                unsigned char *__restrict__ bdr_cell) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nt) return;
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) any |= __ldg(ebdr + __ldg(cedge + 6 * (long)t + k)) != 0;
+  bdr_cell[t] = any ? 1 : 0;
 }
 
 // vslot[t*16 + p*4 + q] = slot of (ctet[t][p], ctet[t][q]) in the vertex pattern
@@ -189,9 +244,13 @@ __global__ void vslot_map_kernel(int nt, const int *__restrict__ tets, const int
 }
 
 void build_slot_maps(Context &c) {
-  c.slot.alloc((size_t)c.nt * 36);
-  long n36 = (long)c.nt * 36;
-  slot_map_kernel<<<(unsigned)((n36 + 255) / 256), 256, 0, c.stream>>>(c.nt, c.cedge.p, c.rp.p, c.ci.p, c.slot.p);
+  if (c.nt >= (1 << kTetBits)) fail(EMG_ERR_ARG, "mesh of %d tets", c.nt);
+  c.erec.alloc((size_t)c.nt * 6);
+  edge_records_kernel<<<(unsigned)((c.ne + 127) / 128), 128, 0, c.stream>>>(c.ne, c.einc_rp.p, c.einc.p, c.cedge.p,
+                                                                            c.ebdr.p, c.rp.p, c.ci.p, c.erec.p);
+  EMG_LAUNCH_CHECK();
+  c.bdr_cell.alloc(c.nt);
+  bdr_cell_kernel<<<(unsigned)((c.nt + 255) / 256), 256, 0, c.stream>>>(c.nt, c.cedge.p, c.ebdr.p, c.bdr_cell.p);
   EMG_LAUNCH_CHECK();
   c.vslot.alloc((size_t)c.nt * 16);
   long n16 = (long)c.nt * 16;
@@ -249,6 +308,12 @@ void canonicalize(Context &c) {
   bad.download(&hb, 1, c.stream);
   EMG_CUDA(cudaStreamSynchronize(c.stream));
   if (hb) fail(EMG_ERR_USER, "tet %d: tet2edgelist does not match tetrahedronlist/edgelist", hb - 1);
+}
+
+__device__ __forceinline__ void cross3(const double *a, const double *b, double *o) {
+  o[0] = a[1] * b[2] - a[2] * b[1];
+  o[1] = a[2] * b[0] - a[0] * b[2];
+  o[2] = a[0] * b[1] - a[1] * b[0];
 }
 
 struct ElemIn {
@@ -319,42 +384,118 @@ __device__ __forceinline__ bool element_matrices(const ElemIn &in, int t, double
   return any;
 }
 
-constexpr int ASM_THREADS = 64;
+// One thread per matrix row: the edge's row of the element matrices of each
+// incident tet, summed in the row's slots of a shared tile and written once.
+// A pair of edges meets in at most two tets (one per side of their common
+// face), only the diagonal in more, so the tet-wise scatter that this
+// replaces spent 72 FP64 atomics per tet on entries with one or two terms and
+// was bound by them.  The row-wise sum recomputes a tet's geometry for each of
+// its six edges instead, needs no atomics, no cleared arrays and no 36-entry
+// slot map per tet, and always sums in the same order.
+// Bound: the gathers of vertices and the FP64 pipe.
+constexpr int ASM_ROWS = 128;
+constexpr int ASM_SLOTS = ASM_ROWS * 18;  // a tile holds rows of 18 slots on average (36.9 KB)
 
-__global__ void __launch_bounds__(ASM_THREADS) assemble_edge_kernel(ElemIn in, int nt, const int *__restrict__ slot,
-                                                                  double *__restrict__ Cv, double *__restrict__ Mv,
-                                                                  unsigned char *__restrict__ bdr_cell) {
-  __shared__ double sc[ASM_THREADS * 36];
-  __shared__ double sm[ASM_THREADS * 36];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t = blockIdx.x * ASM_THREADS + tid;
-  if (t < nt) {
-    double c[36], m[36];
-    TetGeom g;
-    bool bd = element_matrices(in, t, c, m, g);
-    bdr_cell[t] = bd ? 1 : 0;
+__global__ void __launch_bounds__(ASM_ROWS) assemble_edge_kernel(ElemIn in, int ne, const int *__restrict__ inc_rp,
+                                                               const int *__restrict__ inc,
+                                                               const unsigned long long *__restrict__ rec,
+                                                               const int *__restrict__ rp, const int *__restrict__ ci,
+                                                               double *__restrict__ Cv, double *__restrict__ Mv) {
+  __shared__ double tile[2 * ASM_SLOTS];
+  const int r0 = blockIdx.x * ASM_ROWS, r1 = min(ne, r0 + ASM_ROWS), e = r0 + (int)threadIdx.x;
+  const int s0 = __ldg(rp + r0), ns = __ldg(rp + r1) - s0;
+  const bool tiled = ns <= ASM_SLOTS;
+  double *tc = tiled ? tile : Cv + s0, *tm = tiled ? tile + ASM_SLOTS : Mv + s0;
+  for (int i = threadIdx.x; i < ns; i += ASM_ROWS) tc[i] = tm[i] = 0.0;
+  __syncthreads();
+  if (e < ne) {
+    const int kb = __ldg(rp + e), ke = __ldg(rp + e + 1);
+    double *rc = tc + (kb - s0), *rm = tm + (kb - s0);
+    const int j1 = __ldg(inc_rp + e + 1);
+    for (int j = __ldg(inc_rp + e); j < j1; ++j) {
+      const int tk = __ldg(inc + j), t = tk & ((1 << kTetBits) - 1), k = tk >> kTetBits;
+      const unsigned long long rc6 = __ldg(rec + j);
+      const int4 vs = __ldg(reinterpret_cast<const int4 *>(in.ctet) + t);
+      const int p = kEdgeP(k), q = kEdgeQ(k), u = kOther(k, 0), w = kOther(k, 1);
+      auto at = [&](int i) { return i == 0 ? vs.x : (i == 1 ? vs.y : (i == 2 ? vs.z : vs.w)); };
+      const int v[4] = {at(p), at(q), at(u), at(w)};
+      double x[4][3];
 #pragma unroll
-    for (int k = 0; k < 36; ++k) {
-      sc[tid * 36 + k] = c[k];
-      sm[tid * 36 + k] = m[k];
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[i][d] = __ldg(in.pts + 3 * (long)v[i] + d);
+      double e1[3], e2[3], e3[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        e1[d] = x[1][d] - x[0][d];
+        e2[d] = x[2][d] - x[0][d];
+        e3[d] = x[3][d] - x[0][d];
+      }
+      double g[4][3];
+      cross3(e2, e3, g[1]);
+      cross3(e3, e1, g[2]);
+      cross3(e1, e2, g[3]);
+      const double det = e1[0] * g[1][0] + e1[1] * g[1][1] + e1[2] * g[1][2];
+      const double inv = 1.0 / det;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        g[1][d] *= inv;
+        g[2][d] *= inv;
+        g[3][d] *= inv;
+        g[0][d] = -(g[1][d] + g[2][d] + g[3][d]);
+      }
+      // (a, b, c, d) is an odd permutation of the sorted vertices for the edges 1 and 4
+      const double par = (double)__ldg(in.cpar + t) * ((k == 1 || k == 4) ? -1.0 : 1.0);
+      const double vol = par * det / 6.0;
+      const double *sg = in.sig + 9 * (long)__ldg(in.attr + t);
+      double S0[4], S1[4];  // grad l_a . sigma grad l_i and grad l_b . sigma grad l_i
+      {
+        double a0[3], a1[3];  // sigma is symmetric
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          a0[d] = __ldg(sg + d) * g[0][0] + __ldg(sg + 3 + d) * g[0][1] + __ldg(sg + 6 + d) * g[0][2];
+          a1[d] = __ldg(sg + d) * g[1][0] + __ldg(sg + 3 + d) * g[1][1] + __ldg(sg + 6 + d) * g[1][2];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          S0[i] = a0[0] * g[i][0] + a0[1] * g[i][1] + a0[2] * g[i][2];
+          S1[i] = a1[0] * g[i][0] + a1[1] * g[i][1] + a1[2] * g[i][2];
+        }
+      }
+      double cu[3];
+      cross3(g[0], g[1], cu);
+      const double vc = 4.0 * vol / MU, vm = vol / 20.0;
+      const bool row_bdr = (rc6 >> 58) & 1;
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        const int r = l < 3 ? 0 : (l < 5 ? 1 : 2), s = l < 3 ? l + 1 : (l < 5 ? l - 1 : 3);
+        const bool cut = l > 0 && (row_bdr || ((rc6 >> (58 + l)) & 1));
+        double cr[3];
+        cross3(g[r], g[s], cr);
+        double ckl = vc * (cu[0] * cr[0] + cu[1] * cr[1] + cu[2] * cr[2]);
+        double mkl = vm * ((1.0 + (0 == r)) * S1[s] - (1.0 + (0 == s)) * S1[r] - (1.0 + (1 == r)) * S0[s] +
+                           (1.0 + (1 == s)) * S0[r]);
+        if (l >= 1 && l <= 4 && ((rc6 >> (53 + l)) & 1)) {
+          ckl = -ckl;
+          mkl = -mkl;
+        }
+        if (cut) ckl = 0.0;
+        if (cut || row_bdr) mkl = 0.0;
+        int pos = (int)((rc6 >> (9 * l)) & kSearch);
+        if (pos == (int)kSearch) {
+          const int i0 = l < 3 ? p : (l < 5 ? q : u), i1 = l == 0 ? q : (l == 1 || l == 3 ? u : w);
+          pos = find_col(ci, kb, ke, __ldg(in.cedge + 6 * (long)t + kEdgeOf(min(i0, i1), max(i0, i1)))) - kb;
+        }
+        rc[pos] += ckl;
+        rm[pos] += mkl;
+      }
     }
   }
-  __syncwarp();
-  // warp-cooperative scatter over the (tet, entry) pairs of the warp's 32
-  // tets: slot-map reads are coalesced, shared reads conflict-free
-  const int t0 = blockIdx.x * ASM_THREADS + warp * 32;
-  const int nvalid = min(32, nt - t0);
-  const double *wc = sc + warp * 32 * 36;
-  const double *wm = sm + warp * 32 * 36;
-  const int *ws = slot + (long)t0 * 36;
-#pragma unroll 4
-  for (int r = 0; r < 36; ++r) {
-    int p = r * 32 + lane;
-    if (p < nvalid * 36) {
-      int s = __ldg(ws + p);
-      atomicAdd(Cv + s, wc[p]);
-      atomicAdd(Mv + s, wm[p]);
-    }
+  if (!tiled) return;
+  __syncthreads();
+  for (int i = threadIdx.x; i < ns; i += ASM_ROWS) {
+    Cv[s0 + i] = tc[i];
+    Mv[s0 + i] = tm[i];
   }
 }
 
@@ -365,12 +506,8 @@ ElemIn elem_in(Context &c) {
 void assemble_edge(Context &c) {
   c.Cv.alloc(c.nnz);
   c.Msv.alloc(c.nnz);
-  c.bdr_cell.alloc(c.nt);
-  c.Cv.zero(c.stream);
-  c.Msv.zero(c.stream);
-  unsigned blocks = (unsigned)((c.nt + ASM_THREADS - 1) / ASM_THREADS);
-  assemble_edge_kernel<<<blocks, ASM_THREADS, 0, c.stream>>>(elem_in(c), c.nt, c.slot.p, c.Cv.p, c.Msv.p,
-                                                              c.bdr_cell.p);
+  assemble_edge_kernel<<<(unsigned)((c.ne + ASM_ROWS - 1) / ASM_ROWS), ASM_ROWS, 0, c.stream>>>(
+      elem_in(c), c.ne, c.einc_rp.p, c.einc.p, c.erec.p, c.rp.p, c.ci.p, c.Cv.p, c.Msv.p);
   EMG_LAUNCH_CHECK();
 }
 

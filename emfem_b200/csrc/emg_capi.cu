@@ -805,7 +805,9 @@ int emg_destroy_linear_system(emg_context *c) {
   need(c != nullptr, EMG_ERR_ARG, "null context");
   c->Cv.release();
   c->Msv.release();
-  c->slot.release();
+  c->einc.release();
+  c->einc_rp.release();
+  c->erec.release();
   c->vslot.release();
   c->rp.release();
   c->ci.release();

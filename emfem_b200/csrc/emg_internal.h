@@ -249,7 +249,9 @@ struct Context {
   int tidx = -3;
   std::vector<int> h_rp, h_ci;
   long nnz = 0;
-  DBuf<int> rp, ci, slot;          // slot: 36 per tet
+  DBuf<int> rp, ci;
+  DBuf<int> einc_rp, einc;         // tets around each edge (6 per tet in all)
+  DBuf<unsigned long long> erec;   // their records for the assembly (edge_records_kernel)
   DBuf<double> Cv, Msv;            // C and Ms (omega-free mass) on the pattern
   DBuf<unsigned char> bdr_cell;
   bool assembled = false;
@@ -304,7 +306,7 @@ void sigma_table(int aniso_form, int nrho, int ncol, const double *rho, std::vec
 void build_sparsity(Context &c);          // host: CSR pattern (make_sparsity_patterns)
 void build_vertex_pattern(Context &c);    // host: vertex adjacency + incidence
 void canonicalize(Context &c);            // device: sorted tets + canonical edges
-void build_slot_maps(Context &c);         // device: tet -> CSR slots
+void build_slot_maps(Context &c);         // device: edge incidence records, tet -> vertex CSR slots
 void assemble_edge(Context &c);           // device: C, Ms, bdr cells
 void assemble_nodal(Context &c, HCsr out[4]);  // device + download (G, Pi_x, Pi_y, Pi_z)
 // the same on the device only: buf holds 8 vertex-pattern arrays, part p of
