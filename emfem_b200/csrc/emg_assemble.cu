@@ -113,6 +113,7 @@ void build_sparsity(Context &c) {
   }
   c.rp.upload(c.h_rp, c.stream);
   c.ci.upload(c.h_ci, c.stream);
+  c.chunk_rp.release();
   c.einc_rp.upload(e2t_rp, c.stream);
   c.einc.upload(e2t, c.stream);
   EMG_CUDA(cudaStreamSynchronize(c.stream));  // the incidence lists go out of scope

@@ -48,6 +48,85 @@ void launch_check(const char *file, int line) {
   check_cuda(cudaGetLastError(), "kernel launch", file, line);
 }
 
+DevicePool *&current_pool() {
+  static thread_local DevicePool *p = nullptr;
+  return p;
+}
+
+void *DevicePool::get(size_t &bytes) {
+  bytes = (bytes + 511) / 512 * 512;
+  // a block up to an eighth (and 64 KB) larger than asked for
+  auto it = blocks.lower_bound(bytes);
+  if (it != blocks.end() && it->first <= bytes + bytes / 8 + 65536) {
+    void *p = it->second;
+    bytes = it->first;
+    cached -= bytes;
+    blocks.erase(it);
+    return p;
+  }
+  void *p = nullptr;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    if (blocks.empty()) break;
+    trim();
+  }
+  return nullptr;
+}
+
+void DevicePool::put(void *p, size_t bytes) {
+  if (cached + bytes > kPoolKeep) {
+    cudaFree(p);
+    return;
+  }
+  try {
+    blocks.emplace(bytes, p);
+    cached += bytes;
+  } catch (...) {
+    cudaFree(p);
+  }
+}
+
+void DevicePool::trim() {
+  for (auto &b : blocks) cudaFree(b.second);  // waits for the GPU
+  blocks.clear();
+  cached = 0;
+}
+
+PinnedStage::~PinnedStage() {
+  for (int i = 0; i < 2; ++i) {
+    if (buf[i]) cudaFreeHost(buf[i]);
+    if (done[i]) cudaEventDestroy(done[i]);
+  }
+}
+
+void PinnedStage::download(void *host, const void *dev, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return;
+  if (!done[1]) {
+    for (int i = 0; i < 2; ++i) {
+      if (!buf[i]) EMG_CUDA(cudaMallocHost((void **)&buf[i], kBytes));
+      if (!done[i]) EMG_CUDA(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
+    }
+  }
+  const long n = (long)((bytes + kBytes - 1) / kBytes);
+  auto size = [&](long i) { return std::min(kBytes, bytes - (size_t)i * kBytes); };
+  for (long i = 0; i <= n; ++i) {
+    if (i < n) {
+      EMG_CUDA(cudaMemcpyAsync(buf[i & 1], (const char *)dev + (size_t)i * kBytes, size(i), cudaMemcpyDeviceToHost, s));
+      EMG_CUDA(cudaEventRecord(done[i & 1], s));
+    }
+    if (i == 0) continue;
+    EMG_CUDA(cudaEventSynchronize(done[(i - 1) & 1]));
+    char *to = (char *)host + (size_t)(i - 1) * kBytes;
+    const char *from = buf[(i - 1) & 1];
+    const long m = (long)size(i - 1);
+    constexpr long kPart = 64 << 10;
+    const long parts = (m + kPart - 1) / kPart;
+#pragma omp parallel for schedule(static) if (parts > 1)
+    for (long q = 0; q < parts; ++q) std::memcpy(to + q * kPart, from + q * kPart, std::min(kPart, m - q * kPart));
+  }
+}
+
 KernelProfiler &profiler() {
   static KernelProfiler p;
   return p;
@@ -724,6 +803,7 @@ int emg_set_mesh(emg_context *c, int nv, const double *pts, int nt, const int *t
   c->have_pc = false;
   c->ws->block_ready64 = c->ws->block_ready32 = false;
   c->sol.clear();
+  c->pool.trim();
   if (c->device < 0) return EMG_OK;  // host-only context: host-side entry points only
   c->pts.upload(c->h_pts, c->stream);
   c->tets.upload(c->h_tets, c->stream);
@@ -766,16 +846,18 @@ int emg_set_frequencies(emg_context *c, int n, const double *f) {
   EMG_API_END
 }
 
-// makes the context's GPU current; a host-only context (device -1) refuses
-static void use_device(const Context &c) {
+// makes the context's GPU current and its pool the source of allocations
+// while the result lives; a host-only context (device -1) refuses
+static PoolScope use_device(Context &c) {
   need(c.device >= 0, EMG_ERR_STATE, "host-only context has no device");
   EMG_CUDA(cudaSetDevice(c.device));
+  return PoolScope(c.pool);
 }
 
 int emg_create_linear_system(emg_context *c, int tidx) {
   EMG_API_BEGIN
   need(c && c->nt > 0, EMG_ERR_STATE, "create_linear_system before emg_set_mesh");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   c->tidx = tidx;
   c->tiles.clear();
   build_sparsity(*c);
@@ -814,6 +896,8 @@ int emg_destroy_linear_system(emg_context *c) {
   c->sol.clear();
   c->have_ls = c->assembled = c->have_pc = false;
   c->ws->block_ready64 = c->ws->block_ready32 = false;
+  if (c->device >= 0) EMG_CUDA(cudaSetDevice(c->device));
+  c->pool.trim();
   EMG_API_END
 }
 
@@ -832,7 +916,7 @@ int emg_assemble_matrix(emg_context *c, int fidx) {
   need(c && c->have_ls, EMG_ERR_STATE, "assemble_matrix before create_linear_system");
   need(c->nrho > 0, EMG_ERR_STATE, "assemble_matrix before emg_set_model");
   need(fidx >= 0 && fidx < (int)c->freqs.size(), EMG_ERR_ARG, "frequency index out of range");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   c->omega = 2 * PI * c->freqs[fidx];
   cudaEvent_t e0, e1;
   EMG_CUDA(cudaEventCreate(&e0));
@@ -860,7 +944,7 @@ __global__ static void scale_copy_kernel(long n, const double *a, double w, doub
 int emg_get_matrices(emg_context *c, double *C, double *M, unsigned char *bdr) {
   EMG_API_BEGIN
   need(c && c->assembled, EMG_ERR_STATE, "matrices not assembled");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   if (C) c->Cv.download(C, c->nnz, c->stream);
   if (M) {
     DBuf<double> tmp(c->nnz);
@@ -877,7 +961,7 @@ int emg_get_matrices(emg_context *c, double *C, double *M, unsigned char *bdr) {
 int emg_create_pc(emg_context *c) {
   EMG_API_BEGIN
   need(c && c->assembled, EMG_ERR_STATE, "create_pc before assemble_matrix");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   cudaEvent_t e0, e1;
   EMG_CUDA(cudaEventCreate(&e0));
   EMG_CUDA(cudaEventCreate(&e1));
@@ -908,7 +992,7 @@ int emg_matshell_mult_a(emg_context *c, const double *x, double *y) {
   EMG_API_BEGIN
   need(c && x && y, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "operator not assembled");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   const int n = c->ne;
   std::vector<double> xi = interleave(x, x + n, n);
   Workspace &w = *c->ws;
@@ -929,7 +1013,7 @@ int emg_pc_apply_b(emg_context *c, const double *b, double *x) {
   EMG_API_BEGIN
   need(c && b && x, EMG_ERR_ARG, "null argument");
   need(c->have_pc, EMG_ERR_STATE, "pc_apply_b before create_pc");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   const int n = c->ne;
   Workspace &w = *c->ws;
   std::vector<double> bi = interleave(b, b + n, n);
@@ -966,7 +1050,7 @@ int emg_solve_linear_system(emg_context *c, int target, const double *s_re, cons
   need(c && s_re && s_im, EMG_ERR_ARG, "null argument");
   need(c->have_pc, EMG_ERR_STATE, "solve_linear_system before create_pc");
   need(max_it > 0 && rtol > 0, EMG_ERR_ARG, "bad tolerances");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   const int n = c->ne;
   Workspace &w = *c->ws;
   DBuf<double> &x = slot_buf(*c, target);
@@ -997,7 +1081,7 @@ int emg_get_solution(emg_context *c, int target, double *e_re, double *e_im) {
   EMG_API_BEGIN
   need(c && (e_re || e_im), EMG_ERR_ARG, "null argument");
   need(c->have_ls, EMG_ERR_STATE, "no linear system");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   DBuf<double> &x = slot_buf(*c, target);
   std::vector<double> v((size_t)c->ne * 2);
   x.download(v.data(), v.size(), c->stream);
@@ -1013,7 +1097,7 @@ int emg_set_solution(emg_context *c, int target, const double *e_re, const doubl
   EMG_API_BEGIN
   need(c && e_re && e_im, EMG_ERR_ARG, "null argument");
   need(c->have_ls, EMG_ERR_STATE, "no linear system");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   DBuf<double> &x = slot_buf(*c, target);
   std::vector<double> v = interleave(e_re, e_im, c->ne);
   x.upload(v, c->stream);
@@ -1078,7 +1162,7 @@ int emg_assemble_rhs_mt(emg_context *c, int fidx, int mode, double *s_re, double
   need(c->assembled, EMG_ERR_STATE, "assemble_rhs_mt before assemble_matrix");
   need(fidx >= 0 && fidx < (int)c->freqs.size(), EMG_ERR_ARG, "frequency index out of range");
   need(mode == EMG_SOL_MT_XY || mode == EMG_SOL_MT_YX, EMG_ERR_ARG, "mode must be XY_POLAR or YX_POLAR");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   DBuf<double> s((size_t)c->ne * 2);
   double f = c->freqs[fidx];
   rhs_mt_block(*c, 1, &f, &mode, s.p);
@@ -1163,7 +1247,7 @@ int emg_estimate_error(emg_context *c, int fidx, int tidx, double *err, double *
   need(c && (err || eta_raw), EMG_ERR_ARG, "null argument");
   need(c->have_ls && c->nrho > 0, EMG_ERR_STATE, "estimate_error before create_linear_system");
   need(fidx >= 0 && fidx < (int)c->freqs.size(), EMG_ERR_ARG, "frequency index out of range");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   Workspace &w = *c->ws;
   std::vector<int> slots = tidx < 0 ? std::vector<int>{EMG_SOL_MT_XY, EMG_SOL_MT_YX, EMG_SOL_DUAL}
                                     : std::vector<int>{EMG_SOL_CSEM, EMG_SOL_DUAL};
@@ -1180,8 +1264,8 @@ int emg_estimate_error(emg_context *c, int fidx, int tidx, double *err, double *
   EMG_CUDA(cudaEventRecord(e0, c->stream));
   launch_estimate(*c, 2 * PI * c->freqs[fidx], nsol, sp, w.est_eta.p, w.est_err.p, w.est_vol.p, w.est_fe.p);
   EMG_CUDA(cudaEventRecord(e1, c->stream));
-  if (err) w.est_err.download(err, (size_t)(nsol - 1) * c->nt, c->stream);
-  if (eta_raw) w.est_eta.download(eta_raw, (size_t)nsol * c->nt, c->stream);
+  if (err) c->stage.download(err, w.est_err.p, sizeof(double) * (size_t)(nsol - 1) * c->nt, c->stream);
+  if (eta_raw) c->stage.download(eta_raw, w.est_eta.p, sizeof(double) * (size_t)nsol * c->nt, c->stream);
   EMG_CUDA(cudaEventSynchronize(e1));
   float ms = 0;
   EMG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -1269,7 +1353,7 @@ int emg_interpolate_fields(emg_context *c, int target, int fidx, int n, const do
   EMG_API_BEGIN
   need(c && pts && tets && eh, EMG_ERR_ARG, "null argument");
   need(fidx >= 0 && fidx < (int)c->freqs.size(), EMG_ERR_ARG, "frequency index out of range");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   DBuf<double> &x = slot_buf(*c, target);
   // the slot is an n x 1 complex block: the receiver kernel reads only the
   // edges of the receivers' cells
@@ -1808,7 +1892,7 @@ int emg_solve_block_dev(emg_context *c, int k, const double *freqs, const double
                         const emg_block_opts *opts, emg_solve_info *infos) {
   EMG_API_BEGIN
   need(c && freqs && rhs_dev && x_dev && opts, EMG_ERR_ARG, "null argument");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   solve_block_dev(*c, k, freqs, rhs_dev, x_dev, *opts, infos);
   EMG_API_END
 }
@@ -1819,7 +1903,7 @@ int emg_divergence_correct_dev(emg_context *c, int k, const double *freqs, const
   need(c && freqs && rhs_dev && x_dev, EMG_ERR_ARG, "null argument");
   need(k >= 1 && (k & (k - 1)) == 0 && k <= 32, EMG_ERR_ARG, "block width k must be a power of two <= 32");
   need(c->assembled, EMG_ERR_STATE, "divergence correction before assemble_matrix");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   Workspace &w = *c->ws;
   need(fp32 ? w.block_ready32 : w.block_ready64, EMG_ERR_STATE,
        "divergence correction before a block solve of that precision");
@@ -1847,7 +1931,7 @@ int emg_solve_block(emg_context *c, int k, const double *freqs, const double *rh
                     const emg_block_opts *opts, emg_solve_info *infos) {
   EMG_API_BEGIN
   need(c && freqs && rhs && x && opts, EMG_ERR_ARG, "null argument");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   const size_t N = (size_t)c->ne * k * 2;
   DBuf<double> b(N), xd(N);
   b.upload(rhs, N, c->stream);
@@ -1863,7 +1947,7 @@ int emg_spmv_complex_dev(emg_context *c, int k, const double *omegas, const doub
   EMG_API_BEGIN
   need(c && omegas && x_dev && y_dev, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "operator not assembled");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   spmm_complex_host(c->ne, k, c->rp.p, c->ci.p, c->Cv.p, c->Msv.p, omegas, x_dev, y_dev, conj_out != 0, c->stream);
   EMG_API_END
 }
@@ -1874,7 +1958,7 @@ int emg_spmm_layout_dev(emg_context *c, int fp32, int K, int v, int variant, con
   need(c && omegas && x_dev && b_dev && y_dev, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "operator not assembled");
   need(K >= 1 && K <= 64, EMG_ERR_ARG, "block width K out of range");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   cudaStream_t s = c->stream;
   c->ws->omega_k.upload(omegas, K, s);
   SpmmArgs a;
@@ -1939,7 +2023,7 @@ int emg_amg_levels(emg_context *c, int sp, int gpu, double w_ref, int max_rows, 
   need(c && nlev && out, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "AMG levels before assemble_matrix");
   need(sp >= 0 && sp < NSUB, EMG_ERR_ARG, "subspace index out of range");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   std::vector<double> v;
   amg_levels_report(*c, sp, gpu != 0, w_ref, v);
   const int nl = (int)(v.size() / 5);
@@ -2010,7 +2094,7 @@ int emg_assemble_rhs_mt_block_dev(emg_context *c, int k, const double *freqs, co
   need(c->assembled, EMG_ERR_STATE, "assemble_rhs_mt before assemble_matrix");
   for (int j = 0; j < k; ++j)
     need(modes[j] == EMG_SOL_MT_XY || modes[j] == EMG_SOL_MT_YX, EMG_ERR_ARG, "mode must be XY_POLAR or YX_POLAR");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   rhs_mt_block(*c, k, freqs, modes, s_dev);
   EMG_API_END
 }
@@ -2019,7 +2103,7 @@ int emg_assemble_rhs_mt_block(emg_context *c, int k, const double *freqs, const 
   EMG_API_BEGIN
   need(c && freqs && modes && s && k > 0, EMG_ERR_ARG, "null argument");
   need(c->assembled, EMG_ERR_STATE, "assemble_rhs_mt before assemble_matrix");
-  use_device(*c);
+  const PoolScope on = use_device(*c);
   DBuf<double> d((size_t)c->ne * k * 2);
   rhs_mt_block(*c, k, freqs, modes, d.p);
   d.download(s, (size_t)c->ne * k * 2, c->stream);

@@ -114,9 +114,10 @@ __global__ void __launch_bounds__(128) point_source_kernel(const double *pts, co
   }
 }
 
-void device_only(const Context &c) {
+PoolScope device_only(Context &c) {
   need(c.device >= 0, EMG_ERR_STATE, "this entry point needs a device context (device >= 0)");
   EMG_CUDA(cudaSetDevice(c.device));
+  return PoolScope(c.pool);
 }
 
 void launch_point_sources(Context &c, const std::vector<PointSource> &src, int k, double *s_dev) {
@@ -144,7 +145,7 @@ int emg_interpolate_fields_block_dev(emg_context *c, int k, const double *freqs,
   need(c && freqs && x_dev && (n == 0 || (pts && tets && eh)), EMG_ERR_ARG, "null argument");
   need(k >= 1 && n >= 0, EMG_ERR_ARG, "bad block width or receiver count");
   need(c->have_ls, EMG_ERR_STATE, "interpolate_fields before create_linear_system");
-  device_only(*c);
+  const PoolScope on = device_only(*c);
   if (n == 0) return EMG_OK;
   for (int r = 0; r < n; ++r)
     if (tets[r] < 0 || tets[r] >= c->nt) fail(EMG_ERR_USER, "Receiver %d is not found in mesh.", r);
@@ -162,8 +163,7 @@ int emg_interpolate_fields_block_dev(emg_context *c, int k, const double *freqs,
   const long m = (long)n * k;
   fields_block_kernel<<<(unsigned)((m + 127) / 128), 128, 0, c->stream>>>(a);
   EMG_LAUNCH_CHECK();
-  deh.download(eh, (size_t)n * k * 12, c->stream);
-  EMG_CUDA(cudaStreamSynchronize(c->stream));
+  c->stage.download(eh, deh.p, sizeof(double) * (size_t)n * k * 12, c->stream);
   EMG_API_END
 }
 
@@ -172,7 +172,7 @@ int emg_assemble_rhs_csem_block_dev(emg_context *c, int k, const double *freqs, 
   need(c && freqs && tx && s_dev, EMG_ERR_ARG, "null argument");
   need(k >= 1, EMG_ERR_ARG, "bad block width");
   need(c->have_ls, EMG_ERR_STATE, "assemble_rhs_csem before create_linear_system");
-  device_only(*c);
+  const PoolScope on = device_only(*c);
   std::vector<PointSource> src;
   std::vector<double> P;
   std::vector<int> owner;
@@ -226,7 +226,7 @@ int emg_assemble_rhs_dual_block_dev(emg_context *c, int k, int n_rx, const doubl
   need(c && (n_rx == 0 || rx) && s_dev, EMG_ERR_ARG, "null argument");
   need(k >= 1 && n_rx >= 0, EMG_ERR_ARG, "bad block width or receiver count");
   need(c->have_ls, EMG_ERR_STATE, "assemble_rhs_dual before create_linear_system");
-  device_only(*c);
+  const PoolScope on = device_only(*c);
   std::vector<int> cell(n_rx);
   if (n_rx) {
     int rc = emg_find_cell_around_point(c, n_rx, rx, cell.data());

@@ -59,36 +59,86 @@ long launch_count();
 void add_launches(long n);
 
 // ---------------------------------------------------------------------------
-// device buffer (cudaMalloc-backed, move-only)
+// device memory of a context
+// ---------------------------------------------------------------------------
+// Freed blocks are kept for the context's next allocations: cudaMalloc and
+// cudaFree take 0.1 ms each and now and then tens of milliseconds, an AMS
+// setup needs some 150 of them and a receiver call 4.  A block goes straight
+// back to work without waiting for the GPU, because a context's work runs on
+// its one stream.  At most kPoolKeep bytes stay cached; trim() (called when a
+// linear system or its context is destroyed, a mesh is set, or an allocation
+// fails) gives them back.  Used by one thread at a time, like its context.
+struct DevicePool {
+  static constexpr size_t kPoolKeep = size_t(4) << 30;
+  std::multimap<size_t, void *> blocks;  // by size
+  size_t cached = 0;
+  DevicePool() = default;
+  DevicePool(const DevicePool &) = delete;
+  DevicePool &operator=(const DevicePool &) = delete;
+  ~DevicePool() { trim(); }
+  void *get(size_t &bytes);  // at least `bytes` (set to the block's size); null when out of memory
+  void put(void *p, size_t bytes);
+  void trim();
+};
+
+// the pool that allocations of this thread come from (null: cudaMalloc)
+DevicePool *&current_pool();
+struct PoolScope {
+  DevicePool *before;
+  explicit PoolScope(DevicePool &pool) : before(current_pool()) { current_pool() = &pool; }
+  PoolScope(const PoolScope &) = delete;
+  PoolScope &operator=(const PoolScope &) = delete;
+  ~PoolScope() { current_pool() = before; }
+};
+
+// ---------------------------------------------------------------------------
+// device buffer (from the current pool or cudaMalloc, move-only)
 // ---------------------------------------------------------------------------
 template <typename T>
 struct DBuf {
   T *p = nullptr;
   size_t n = 0;
+  DevicePool *pool = nullptr;  // where the block came from
+  size_t block = 0;            // its size
   DBuf() = default;
   explicit DBuf(size_t count) { alloc(count); }
   DBuf(const DBuf &) = delete;
   DBuf &operator=(const DBuf &) = delete;
-  DBuf(DBuf &&o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+  DBuf(DBuf &&o) noexcept { take(o); }
   DBuf &operator=(DBuf &&o) noexcept {
-    if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+    if (this != &o) {
+      release();
+      take(o);
+    }
     return *this;
   }
   ~DBuf() { release(); }
+  void take(DBuf &o) noexcept {
+    p = o.p;
+    n = o.n;
+    pool = o.pool;
+    block = o.block;
+    o.p = nullptr;
+    o.n = 0;
+  }
   void alloc(size_t count) {
     if (count == n && p) return;
     release();
     if (count == 0) return;
-    cudaError_t e = cudaMalloc((void **)&p, count * sizeof(T));
-    if (e != cudaSuccess) {
+    pool = current_pool();
+    block = count * sizeof(T);
+    if (pool) {
+      p = static_cast<T *>(pool->get(block));
+    } else if (cudaMalloc((void **)&p, block) != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
-      fail(EMG_ERR_NOMEM, "device allocation of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
     }
+    if (!p) fail(EMG_ERR_NOMEM, "device allocation of %zu bytes failed", count * sizeof(T));
     n = count;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && pool) pool->put(p, block);
+    else if (p) cudaFree(p);
     p = nullptr;
     n = 0;
   }
@@ -110,6 +160,21 @@ struct DBuf {
     if (n) EMG_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }
   size_t bytes() const { return n * sizeof(T); }
+};
+
+// Copies device results to pageable host memory through two pinned buffers: the
+// GPU fills one while the host's threads empty the other.  The driver's own
+// copy to pageable memory goes through one thread (12 MB of error indicators:
+// 1.5 ms).  Returns when host[0 .. bytes) is written.
+struct PinnedStage {
+  static constexpr size_t kBytes = size_t(2) << 20;  // each buffer
+  char *buf[2] = {nullptr, nullptr};
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  PinnedStage() = default;
+  PinnedStage(const PinnedStage &) = delete;
+  PinnedStage &operator=(const PinnedStage &) = delete;
+  ~PinnedStage();
+  void download(void *host, const void *dev, size_t bytes, cudaStream_t s);
 };
 
 // host CSR
@@ -220,6 +285,8 @@ struct Workspace;
 // context (mirrors EMContext, em_ctx.h:15-64)
 // ---------------------------------------------------------------------------
 struct Context {
+  DevicePool pool;  // first member: outlives every buffer below
+  PinnedStage stage;
   int device = 0;
   cudaStream_t stream = nullptr;
   Options opt;
@@ -250,6 +317,8 @@ struct Context {
   std::vector<int> h_rp, h_ci;
   long nnz = 0;
   DBuf<int> rp, ci;
+  DBuf<int> chunk_rp;              // chunk row pointer of the pattern (SpmmArgs::crp), built on first use
+  long n_chunks = 0;
   DBuf<int> einc_rp, einc;         // tets around each edge (6 per tet in all)
   DBuf<unsigned long long> erec;   // their records for the assembly (edge_records_kernel)
   DBuf<double> Cv, Msv;            // C and Ms (omega-free mass) on the pattern

@@ -44,6 +44,17 @@ __global__ void l1_rowsum_kernel(int n, const int *__restrict__ rp, const double
   out[i] = (T)s;
 }
 
+// edge tangents x(v1) - x(v0)
+template <typename T>
+__global__ void edge_tangent_kernel(long n, const int *__restrict__ edges, const double *__restrict__ pts,
+                                    T *__restrict__ out) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long e = i / 3;
+  const int d = (int)(i - 3 * e);
+  out[i] = (T)(pts[3 * (long)edges[2 * e + 1] + d] - pts[3 * (long)edges[2 * e] + d]);
+}
+
 template <typename T>
 static void convert(const std::vector<double> &a, std::vector<T> &b) {
   b.resize(a.size());
@@ -229,27 +240,24 @@ void ams_setup(Context &c, Ams<T> &ams, bool per_frequency, double w, double w_r
   if (sizeof(T) == 4 && !per_frequency) {
     ams.Bpk.alloc(c.nnz);
     pack_records(c.nnz, c.ci.p, (const float *)ams.B.vc.p, (const float *)ams.B.vm.p, ams.Bpk.p, s);
-    std::vector<int> crp;
-    const long nch = chunk_row_pointer(c.h_rp, crp);
-    ams.Bcrp.upload(crp, s);
-    ams.Bch.alloc((size_t)std::max(3 * nch, 3L));
-    chunk_records(c.ne, c.rp.p, c.ci.p, (const float *)ams.B.vc.p, (const float *)ams.B.vm.p, ams.Bcrp.p,
-                  ams.Bch.p, s);
-    EMG_CUDA(cudaStreamSynchronize(s));  // the host row pointer goes out of scope
+    if (!c.chunk_rp.p) {  // once per pattern
+      std::vector<int> crp;
+      c.n_chunks = chunk_row_pointer(c.h_rp, crp);
+      c.chunk_rp.upload(crp, s);
+      EMG_CUDA(cudaStreamSynchronize(s));  // the host row pointer goes out of scope
+    }
+    ams.bcrp = c.chunk_rp.p;
+    ams.Bch.alloc((size_t)std::max(3 * c.n_chunks, 3L));
+    chunk_records(c.ne, c.rp.p, c.ci.p, (const float *)ams.B.vc.p, (const float *)ams.B.vm.p, ams.bcrp, ams.Bch.p, s);
   } else {
     ams.Bpk.release();
     ams.Bch.release();
-    ams.Bcrp.release();
+    ams.bcrp = nullptr;
   }
-  // edge tangents x(v1) - x(v0)
-  {
-    std::vector<T> tg((size_t)c.ne * 3);
-    for (int e = 0; e < c.ne; ++e)
-      for (int d = 0; d < 3; ++d)
-        tg[3 * (size_t)e + d] = (T)(c.h_pts[3 * (size_t)c.h_edges[2 * e + 1] + d] - c.h_pts[3 * (size_t)c.h_edges[2 * e] + d]);
-    ams.tangent.upload(tg, s);
-    EMG_CUDA(cudaStreamSynchronize(s));
-  }
+  ams.tangent.alloc((size_t)c.ne * 3);
+  edge_tangent_kernel<T><<<(unsigned)((3L * c.ne + 255) / 256), 256, 0, s>>>(3L * c.ne, c.edges.p, c.pts.p,
+                                                                             ams.tangent.p);
+  EMG_LAUNCH_CHECK();
   EMG_CUDA(cudaStreamSynchronize(s));
   clk.lap("setup_edge");
   // G^T B for the gradient-space residual
@@ -480,7 +488,7 @@ void Ams<T>::spmm_B(int mode, const T *x, const T *b, T *y, cudaStream_t s) {
   std::memset(&a, 0, sizeof(a));
   a.pk = Bpk.p;
   a.ch = Bch.p;
-  a.crp = Bcrp.p;
+  a.crp = bcrp;
   a.n = ne;
   a.rp = brp;
   a.ci = bci;
@@ -636,7 +644,7 @@ T *Ams<T>::smooth(const DCsr<T> *A, long nnz, int n, T *cur, T *oth, const T *b,
     std::memset(&a, 0, sizeof(a));
     a.pk = edge ? Bpk.p : nullptr;
     a.ch = edge ? Bch.p : nullptr;
-    a.crp = edge ? Bcrp.p : nullptr;
+    a.crp = edge ? bcrp : nullptr;
     a.n = n;
     a.rp = edge ? brp : A->rp.p;
     a.ci = edge ? bci : A->ci.p;

@@ -119,12 +119,17 @@ std::vector<Spec> training_specs(const std::vector<Column> &cols) {
   return specs;
 }
 
-void prepare(Context &c, WarmStartNet &net, unsigned seed) {
+// the scope of the context's pool for the rest of the call
+PoolScope prepare(Context &c, WarmStartNet &net, unsigned seed) {
   need(c.device >= 0, EMG_ERR_STATE, "the warm start needs a device context");
   need(c.have_ls && c.nrho > 0, EMG_ERR_STATE, "warm start before create_linear_system and emg_set_model");
   EMG_CUDA(cudaSetDevice(c.device));
-  if (!net.ready) net.init(seed, c.stream);
-  if (net.stat_ne != c.ne || !net.stat.p) net.statics(c);
+  {
+    const PoolScope on(c.pool);
+    if (!net.ready) net.init(seed, c.stream);
+    if (net.stat_ne != c.ne || !net.stat.p) net.statics(c);
+  }
+  return PoolScope(c.pool);
 }
 
 }  // namespace
@@ -142,7 +147,7 @@ int emg_warm_start_train(emg_context *c, int k, const double *freqs, const int *
   need(k >= 2, EMG_ERR_ARG, "training needs at least two solved columns");
   need(o->steps >= 0 && o->batch >= 128 && o->lr > 0, EMG_ERR_ARG, "bad training options");
   WarmStartNet &net = net_of(*c);
-  prepare(*c, net, o->seed);
+  const PoolScope on = prepare(*c, net, o->seed);
   std::vector<Column> cols = columns(k, freqs, src, src_pos);
   std::vector<Spec> specs = training_specs(cols);
   need(!specs.empty(), EMG_ERR_ARG, "no solved column has a solved neighbour of the same source");
@@ -173,7 +178,7 @@ int emg_warm_start_predict(emg_context *c, int k, const double *freqs, const int
   need(c && freqs && x_dev && tfreqs && guess_dev, EMG_ERR_ARG, "null argument");
   need(k >= 1 && kt >= 1, EMG_ERR_ARG, "bad block widths");
   WarmStartNet &net = net_of(*c);
-  prepare(*c, net, 1u);
+  const PoolScope on = prepare(*c, net, 1u);
   std::vector<Column> cols = columns(k, freqs, src, src_pos);
   std::vector<Column> tg = columns(kt, tfreqs, tsrc, tsrc_pos);
   std::vector<Spec> specs;
@@ -235,7 +240,7 @@ int emg_warm_start_params(emg_context *c, float *get, const float *set, int *npa
   if (nparam) *nparam = WarmStartNet::nparam();
   if (!get && !set) return EMG_OK;
   WarmStartNet &net = net_of(*c);
-  prepare(*c, net, 1u);
+  const PoolScope on = prepare(*c, net, 1u);
   if (set) net.set_params(set, c->stream);
   if (get) net.params.download(get, WarmStartNet::nparam(), c->stream);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
@@ -248,7 +253,7 @@ int emg_warm_start_gradients(emg_context *c, int k, const double *freqs, const i
   need(c && freqs && x_dev && grads, EMG_ERR_ARG, "null argument");
   need(batch >= 1 && step >= 0, EMG_ERR_ARG, "bad batch or step");
   WarmStartNet &net = net_of(*c);
-  prepare(*c, net, 1u);
+  const PoolScope on = prepare(*c, net, 1u);
   std::vector<Column> cols = columns(k, freqs, src, src_pos);
   std::vector<Spec> specs = training_specs(cols);
   need(!specs.empty(), EMG_ERR_ARG, "no solved column has a solved neighbour of the same source");
