@@ -93,21 +93,47 @@ void DevicePool::trim() {
   cached = 0;
 }
 
-PinnedStage::~PinnedStage() {
+PinnedStage::PinnedStage() {
   for (int i = 0; i < 2; ++i) {
-    if (buf[i]) cudaFreeHost(buf[i]);
-    if (done[i]) cudaEventDestroy(done[i]);
+    const cudaError_t e = cudaHostAlloc((void **)&buf[i], kBytes, cudaHostAllocPortable);
+    if (e == cudaSuccess) continue;
+    buf[i] = nullptr;
+    if (i) cudaFreeHost(buf[0]);
+    EMG_CUDA(e);
   }
 }
 
-void PinnedStage::download(void *host, const void *dev, size_t bytes, cudaStream_t s) {
+PinnedStage::~PinnedStage() {
+  for (int i = 0; i < 2; ++i)
+    if (buf[i]) cudaFreeHost(buf[i]);
+}
+
+std::shared_ptr<PinnedStage> PinnedStage::get() {
+  static std::mutex mu;
+  static std::weak_ptr<PinnedStage> shared;
+  std::lock_guard<std::mutex> lock(mu);
+  std::shared_ptr<PinnedStage> p = shared.lock();
+  if (!p) shared = p = std::make_shared<PinnedStage>();
+  return p;
+}
+
+StagedCopy::~StagedCopy() {
+  for (int i = 0; i < 2; ++i)
+    if (done[i]) cudaEventDestroy(done[i]);
+}
+
+void StagedCopy::open() {
+  if (!stage) stage = PinnedStage::get();
+  for (int i = 0; i < 2; ++i)
+    if (!done[i]) EMG_CUDA(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
+}
+
+void StagedCopy::download(void *host, const void *dev, size_t bytes, cudaStream_t s) {
   if (bytes == 0) return;
-  if (!done[1]) {
-    for (int i = 0; i < 2; ++i) {
-      if (!buf[i]) EMG_CUDA(cudaMallocHost((void **)&buf[i], kBytes));
-      if (!done[i]) EMG_CUDA(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
-    }
-  }
+  open();
+  std::lock_guard<std::mutex> lock(stage->mu);
+  constexpr size_t kBytes = PinnedStage::kBytes;
+  char *const *buf = stage->buf;
   const long n = (long)((bytes + kBytes - 1) / kBytes);
   auto size = [&](long i) { return std::min(kBytes, bytes - (size_t)i * kBytes); };
   for (long i = 0; i <= n; ++i) {
@@ -121,8 +147,10 @@ void PinnedStage::download(void *host, const void *dev, size_t bytes, cudaStream
     const char *from = buf[(i - 1) & 1];
     const long m = (long)size(i - 1);
     constexpr long kPart = 64 << 10;
+    constexpr size_t kOmpBytes = 1 << 20;
     const long parts = (m + kPart - 1) / kPart;
-#pragma omp parallel for schedule(static) if (parts > 1)
+    // waking the host threads pays from about a megabyte on
+#pragma omp parallel for schedule(static) if (bytes > kOmpBytes)
     for (long q = 0; q < parts; ++q) std::memcpy(to + q * kPart, from + q * kPart, std::min(kPart, m - q * kPart));
   }
 }
@@ -184,7 +212,7 @@ void check_cuda(cudaError_t e, const char *what, const char *file, int line) {
 
 // launchers defined in emg_estimate.cu
 void launch_estimate(Context &c, double omega, int nsol, const double *const *sol_dev, double *eta_dev,
-                     double *err_dev, double *scratch_vol, double *scratch_fe);
+                     double *err_dev, double *scratch_fe);
 void launch_rhs_mt(Context &c, int k, const double *omega_dev, const double *bv_dev, const int *brank_dev,
                    double *s_dev);
 
@@ -193,7 +221,7 @@ struct Workspace {
   Fgmres gm;
   DBuf<double> vec_a, vec_b;       // host<->device staging of complex block vectors
   DBuf<float> f_in, f_out;         // FP32 inner vectors
-  DBuf<double> est_vol, est_fe, est_eta, est_err;
+  DBuf<double> est_fe, est_eta, est_err;
   DBuf<double> bvals, omega_k, omega_cols;
   DBuf<double> blk_rhs, blk_x;     // one padded block of a wider or ragged solve
   // plain path: hierarchy of B(w) for the assembled frequency (create_pc)
@@ -684,6 +712,7 @@ int emg_create_context(emg_context **ctx, int device) {
     // the allocation-free estimator's scratch address, looked up now so that
     // its module is loaded and the address cached before any run
     (void)noalloc_scratch_address(device);
+    c->stage.open();
   } catch (...) {
     delete c;
     throw;
@@ -814,6 +843,7 @@ int emg_set_mesh(emg_context *c, int nv, const double *pts, int nt, const int *t
   c->non.upload(c->h_non, c->stream);
   c->ebdr.upload(c->h_ebdr, c->stream);
   canonicalize(*c);
+  build_faces(*c);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
   EMG_API_END
 }
@@ -1254,7 +1284,6 @@ int emg_estimate_error(emg_context *c, int fidx, int tidx, double *err, double *
   int nsol = (int)slots.size();
   const double *sp[3];
   for (int s = 0; s < nsol; ++s) sp[s] = slot_buf(*c, slots[s]).p;
-  w.est_vol.alloc((size_t)nsol * c->nt);
   w.est_fe.alloc((size_t)nsol * c->nt * 4);
   w.est_eta.alloc((size_t)nsol * c->nt);
   w.est_err.alloc((size_t)(nsol - 1) * c->nt);
@@ -1262,7 +1291,7 @@ int emg_estimate_error(emg_context *c, int fidx, int tidx, double *err, double *
   EMG_CUDA(cudaEventCreate(&e0));
   EMG_CUDA(cudaEventCreate(&e1));
   EMG_CUDA(cudaEventRecord(e0, c->stream));
-  launch_estimate(*c, 2 * PI * c->freqs[fidx], nsol, sp, w.est_eta.p, w.est_err.p, w.est_vol.p, w.est_fe.p);
+  launch_estimate(*c, 2 * PI * c->freqs[fidx], nsol, sp, w.est_eta.p, w.est_err.p, w.est_fe.p);
   EMG_CUDA(cudaEventRecord(e1, c->stream));
   if (err) c->stage.download(err, w.est_err.p, sizeof(double) * (size_t)(nsol - 1) * c->nt, c->stream);
   if (eta_raw) c->stage.download(eta_raw, w.est_eta.p, sizeof(double) * (size_t)nsol * c->nt, c->stream);

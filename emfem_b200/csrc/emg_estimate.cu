@@ -16,6 +16,7 @@
 
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "emg_internal.h"
 #include "emg_kernels.cuh"
@@ -32,50 +33,6 @@ struct EstIn {
   double omega;
 };
 
-__device__ __forceinline__ void load_coef(const EstIn &in, const TetGeom &g, int s, double ur[6], double ui[6]) {
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    double2 v = __ldg(in.sol[s] + g.ge[k]);
-    ur[k] = v.x;
-    ui[k] = v.y;
-  }
-}
-
-// e(x) at barycentric coordinates lam (sorted-vertex order)
-__device__ __forceinline__ void field_at(const TetGeom &g, const double lam[4], const double ur[6],
-                                         const double ui[6], double er[3], double ei[3]) {
-#pragma unroll
-  for (int d = 0; d < 3; ++d) { er[d] = 0; ei[d] = 0; }
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const int p = kEdgeP(k), q = kEdgeQ(k);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double phi = lam[p] * g.gr[q][d] - lam[q] * g.gr[p][d];
-      er[d] = fma(ur[k], phi, er[d]);
-      ei[d] = fma(ui[k], phi, ei[d]);
-    }
-  }
-}
-
-__device__ __forceinline__ void curl_of(const TetGeom &g, const double ur[6], const double ui[6], double cr[3],
-                                        double ci[3]) {
-#pragma unroll
-  for (int d = 0; d < 3; ++d) { cr[d] = 0; ci[d] = 0; }
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const int a = kEdgeP(k), b = kEdgeQ(k);
-    double cu[3] = {2.0 * (g.gr[a][1] * g.gr[b][2] - g.gr[a][2] * g.gr[b][1]),
-                    2.0 * (g.gr[a][2] * g.gr[b][0] - g.gr[a][0] * g.gr[b][2]),
-                    2.0 * (g.gr[a][0] * g.gr[b][1] - g.gr[a][1] * g.gr[b][0])};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      cr[d] = fma(ur[k], cu[d], cr[d]);
-      ci[d] = fma(ui[k], cu[d], ci[d]);
-    }
-  }
-}
-
 __device__ __forceinline__ void load_sigma(const EstIn &in, int t, double s[9]) {
   const double *sg = in.sig + 9 * (long)__ldg(in.attr + t);
 #pragma unroll
@@ -87,12 +44,169 @@ __device__ __forceinline__ double dist3(const double *a, const double *b) {
   return sqrt(dx * dx + dy * dy + dz * dz);
 }
 
-__device__ __forceinline__ double sel4(int p, double a0, double a1, double a2, double a3) {
-  return p == 0 ? a0 : (p == 1 ? a1 : (p == 2 ? a2 : a3));
+__device__ __forceinline__ void cmad(double2 &a, double f, double2 u) {  // a += f u
+  a.x = fma(f, u.x, a.x);
+  a.y = fma(f, u.y, a.y);
 }
 
-// vol[s*T + t] = volume term of tet t (integrate_over_cell)
-__global__ void __launch_bounds__(128) estimate_cell_kernel(EstIn in, int nt, double *__restrict__ vol) {
+// One side of a face: the tet's vertices in the order a < b < c of the face's
+// global ids, then the opposite vertex o.
+struct FaceSide {
+  double g[4][3];  // barycentric gradients
+  double h[4];     // g_i . (sigma^T n): normal current of the unit gradient
+  double m[4];     // g_i . n
+  int eo[3];       // edges (a, o), (b, o), (c, o)
+  double so[3];    // +1 where the edge runs towards o
+};
+
+// canonical edge joining sorted positions i < j
+__device__ __forceinline__ int edge_of(int i, int j) { return i == 0 ? j - 1 : (i == 1 ? j + 1 : 5); }
+__device__ __forceinline__ int at4(const int4 &v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
+
+// gradients of tet t seen from its face opposite sorted position p; x: the
+// vertices (a, b, c, o); returns the determinant of the ordered tet
+__device__ __forceinline__ double face_side(const EstIn &in, int t, const int4 &v, int p, double x[4][3], FaceSide &f) {
+  const int q[4] = {p == 0 ? 1 : 0, p <= 1 ? 2 : 1, p <= 2 ? 3 : 2, p};
+  const int vo = at4(v, p);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int vi = at4(v, q[i]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x[i][d] = __ldg(in.pts + 3 * (long)vi + d);
+    if (i < 3) {
+      f.eo[i] = __ldg(in.cedge + 6 * (long)t + edge_of(min(q[i], p), max(q[i], p)));
+      f.so[i] = vi < vo ? 1.0 : -1.0;
+    }
+  }
+  double e1[3], e2[3], e3[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    e1[d] = x[1][d] - x[0][d];
+    e2[d] = x[2][d] - x[0][d];
+    e3[d] = x[3][d] - x[0][d];
+  }
+  const double c23[3] = {e2[1] * e3[2] - e2[2] * e3[1], e2[2] * e3[0] - e2[0] * e3[2], e2[0] * e3[1] - e2[1] * e3[0]};
+  const double c31[3] = {e3[1] * e1[2] - e3[2] * e1[1], e3[2] * e1[0] - e3[0] * e1[2], e3[0] * e1[1] - e3[1] * e1[0]};
+  const double c12[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2], e1[0] * e2[1] - e1[1] * e2[0]};
+  const double det = e1[0] * c23[0] + e1[1] * c23[1] + e1[2] * c23[2], inv = 1.0 / det;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    f.g[1][d] = c23[d] * inv;
+    f.g[2][d] = c31[d] * inv;
+    f.g[3][d] = c12[d] * inv;
+    f.g[0][d] = -(f.g[1][d] + f.g[2][d] + f.g[3][d]);
+  }
+  return det;
+}
+
+__device__ __forceinline__ void face_weights(const EstIn &in, int t, const double n[3], FaceSide &f) {
+  double s[9];
+  load_sigma(in, t, s);
+  double sn[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) sn[d] = s[d] * n[0] + s[3 + d] * n[1] + s[6 + d] * n[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f.h[i] = f.g[i][0] * sn[0] + f.g[i][1] * sn[1] + f.g[i][2] * sn[2];
+    f.m[i] = f.g[i][0] * n[0] + f.g[i][1] * n[1] + f.g[i][2] * n[2];
+  }
+}
+
+// Adds sign times the side's normal current at the face's three vertices to j
+// and its curl x n to c, from the face's edge values (ab, ac, bc) and the
+// three to the opposite vertex.  At vertex a only the edges that end there
+// count: phi_(p,q) = l_p grad l_q - l_q grad l_p; and (g_p x g_q) x n =
+// g_q (g_p . n) - g_p (g_q . n).
+__device__ __forceinline__ void face_terms(const FaceSide &f, const double2 uf[3], const double2 uo[3], double sign,
+                                           double2 j[3], double2 c[3]) {
+  double2 v[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  auto edge = [&](int p, int q, double2 u, double s) {
+    if (p < 3) cmad(j[p], sign * s * f.h[q], u);
+    if (q < 3) cmad(j[q], -sign * s * f.h[p], u);
+    cmad(v[q], s * f.m[p], u);
+    cmad(v[p], -s * f.m[q], u);
+  };
+  edge(0, 1, uf[0], 1.0);
+  edge(0, 2, uf[1], 1.0);
+  edge(1, 2, uf[2], 1.0);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) edge(i, 3, uo[i], f.so[i]);
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cmad(c[d], 2.0 * sign * f.g[i][d], v[i]);
+}
+
+// One thread per interior face (faces[i] = 4 t + f with t the lower tet): both
+// tets' jumps, written to fe[(s*T + t)*4 + f] of both (integrate_over_face).
+// The normal current is linear on the face, so its values at the three
+// vertices give it at the quadrature points (1/2 of the vertex they are near
+// plus 1/6 of all three), and the edges of the face belong to both tets: the
+// kernel needs no quadrature points, no basis functions and 9 edge values.
+// Bound: FP64 and the gathers; nothing spills (it evaluated both fields at
+// three points, spilled 1.1 KB per thread, and half its threads, one per (tet,
+// face), left at once).
+__global__ void __launch_bounds__(128) estimate_face_kernel(EstIn in, int nt, int nfaces,
+                                                            const int *__restrict__ faces, double *__restrict__ fe) {
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= nfaces) return;
+  const int id = __ldg(faces + i), t = id >> 2;
+  const int n = __ldg(in.nbr + id), non = __ldg(in.non + id);
+  const int4 vt = __ldg(reinterpret_cast<const int4 *>(in.ctet) + t);
+  const int4 vn = __ldg(reinterpret_cast<const int4 *>(in.ctet) + n);
+  const int ot = __ldg(in.tets + id), on = __ldg(in.tets + 4 * (long)n + non);
+  const int p = ot == vt.x ? 0 : (ot == vt.y ? 1 : (ot == vt.z ? 2 : 3));
+  const int pn = on == vn.x ? 0 : (on == vn.y ? 1 : (on == vn.z ? 2 : 3));
+  FaceSide a, b;
+  double nrm[3], jxw, fd;
+  {
+    double x[4][3];
+    const double det = face_side(in, t, vt, p, x, a);
+    // outward normal -grad(l_o)/|grad(l_o)| and the reference's face weight
+    const double gl = sqrt(a.g[3][0] * a.g[3][0] + a.g[3][1] * a.g[3][1] + a.g[3][2] * a.g[3][2]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) nrm[d] = -a.g[3][d] / gl;
+    jxw = gl * fabs(det);
+    // circumradius of the face (src/em_mesh.h:256-274)
+    const double la = dist3(x[1], x[2]), lb = dist3(x[0], x[2]), lc = dist3(x[0], x[1]);
+    const double area = 0.25 * sqrt((la + lb + lc) * (lb + lc - la) * (lc + la - lb) * (la + lb - lc));
+    fd = la * lb * lc / (4.0 * area);
+    face_side(in, n, vn, pn, x, b);
+  }
+  face_weights(in, t, nrm, a);
+  face_weights(in, n, nrm, b);
+  const int qa = p == 0 ? 1 : 0, qb = p <= 1 ? 2 : 1, qc = p <= 2 ? 3 : 2;
+  const int ef[3] = {__ldg(in.cedge + 6 * (long)t + edge_of(qa, qb)), __ldg(in.cedge + 6 * (long)t + edge_of(qa, qc)),
+                     __ldg(in.cedge + 6 * (long)t + edge_of(qb, qc))};
+#pragma unroll 1
+  for (int s = 0; s < in.nsol; ++s) {
+    const double2 *u = in.sol[s];
+    const double2 uf[3] = {__ldg(u + ef[0]), __ldg(u + ef[1]), __ldg(u + ef[2])};
+    const double2 ua[3] = {__ldg(u + a.eo[0]), __ldg(u + a.eo[1]), __ldg(u + a.eo[2])};
+    const double2 ub[3] = {__ldg(u + b.eo[0]), __ldg(u + b.eo[1]), __ldg(u + b.eo[2])};
+    double2 j[3] = {{0, 0}, {0, 0}, {0, 0}}, c[3] = {{0, 0}, {0, 0}, {0, 0}};
+    face_terms(a, uf, ua, 1.0, j, c);
+    face_terms(b, uf, ub, -1.0, j, c);
+    const double tx = (j[0].x + j[1].x + j[2].x) / 6.0, ty = (j[0].y + j[1].y + j[2].y) / 6.0;
+    double v = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double jr = 0.5 * j[q].x + tx, ji = 0.5 * j[q].y + ty;
+      v += jr * jr + ji * ji + 3.0 * (c[q].x * c[q].x + c[q].y * c[q].y);
+    }
+    v *= jxw * fd / 2.0;
+    fe[((long)s * nt + t) * 4 + (id & 3)] = v;
+    fe[((long)s * nt + n) * 4 + non] = v;
+  }
+}
+
+// eta[s][t] = volume term (integrate_over_cell) + the four face terms in the
+// reference's order, then the primal x dual combination sqrt(eta_p * eta_d)
+// (src/em_fwd.cc:1172-1177).  The field at a quadrature point is B times the
+// sum of its values at the four vertices plus (A - B) times the value at the
+// vertex the point is near.
+__global__ void __launch_bounds__(128) estimate_cell_kernel(EstIn in, int nt, const double *__restrict__ fe,
+                                                            double *__restrict__ eta, double *__restrict__ err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   TetGeom g;
@@ -109,145 +223,80 @@ __global__ void __launch_bounds__(128) estimate_cell_kernel(EstIn in, int nt, do
     diam = sqrt(sh * (sh - la) * (sh - lb) * (sh - lc)) / (6.0 * g.vol);
   }
   const double A = 0.585410196624969, B = 0.138196601125011;
-  const double jxw_c = g.vol * 6.0 / 24.0;  // det(J) * 1/24
-  const double w2 = in.omega * in.omega;
-#pragma unroll 1
-  for (int s = 0; s < in.nsol; ++s) {
-    double ur[6], ui[6];
-    load_coef(in, g, s, ur, ui);
-    double res = 0;
+  const double w = in.omega * in.omega * (g.vol * 6.0 / 24.0) * diam * diam;  // omega^2 det(J)/24 R^2
+  const int4 nb = __ldg(reinterpret_cast<const int4 *>(in.nbr) + t);
+  double es[3] = {0, 0, 0};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double lam[4];
+  for (int s = 0; s < 3; ++s) {
+    if (s >= in.nsol) break;
+    // sigma e at the four vertices: the edges that end there
+    double2 y[4][3], sum[3] = {{0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
-      for (int p = 0; p < 4; ++p) lam[p] = (p == q) ? A : B;
-      double er[3], ei[3];
-      field_at(g, lam, ur, ui, er, ei);
-      double sq = 0;
+    for (int p = 0; p < 4; ++p)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        double yr = sg[3 * d] * er[0] + sg[3 * d + 1] * er[1] + sg[3 * d + 2] * er[2];
-        double yi = sg[3 * d] * ei[0] + sg[3 * d + 1] * ei[1] + sg[3 * d + 2] * ei[2];
-        sq += w2 * (yr * yr + yi * yi);
-      }
-      res += sq * jxw_c;
-    }
-    vol[(long)s * nt + t] = res * diam * diam;
-  }
-}
-
-// fe[(s*T + t)*4 + f]: face f (input index) of tet t, evaluated by the lower
-// of the two tets (integrate_over_face)
-__global__ void __launch_bounds__(128) estimate_face_kernel(EstIn in, int nt, double *__restrict__ fe) {
-  const long id = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (id >= (long)nt * 4) return;
-  const int t = (int)(id >> 2), f = (int)(id & 3);
-  const int n = __ldg(in.nbr + id);
-  if (n < 0) {
-    for (int s = 0; s < in.nsol; ++s) fe[((long)s * nt + t) * 4 + f] = 0.0;
-    return;
-  }
-  if (n < t) return;  // the neighbour evaluates this face
-  const int non = __ldg(in.non + id);
-  TetGeom g;
-  load_tet_geom(in.pts, in.ctet, in.cedge, in.cpar, t, g);
-  // sorted position of the vertex opposite face f
-  const int vf = __ldg(in.tets + 4 * (long)t + f);
-  const int p = vf == g.v[0] ? 0 : (vf == g.v[1] ? 1 : (vf == g.v[2] ? 2 : 3));
-  double sg[9];
-  load_sigma(in, t, sg);
-  // outward normal -grad(l_p)/|grad(l_p)| and the reference's face weight
-  const double gx = sel4(p, g.gr[0][0], g.gr[1][0], g.gr[2][0], g.gr[3][0]);
-  const double gy = sel4(p, g.gr[0][1], g.gr[1][1], g.gr[2][1], g.gr[3][1]);
-  const double gz = sel4(p, g.gr[0][2], g.gr[1][2], g.gr[2][2], g.gr[3][2]);
-  const double gl = sqrt(gx * gx + gy * gy + gz * gz);
-  const double nrm[3] = {-gx / gl, -gy / gl, -gz / gl};
-  const double jxw_f = gl * fabs(6.0 * g.vol) * 6.0 / 6.0;
-  // face circumradius (src/em_mesh.h:256-274): edge lengths of the face
-  double fd;
-  {
-    double d01 = dist3(g.x[0], g.x[1]), d02 = dist3(g.x[0], g.x[2]), d03 = dist3(g.x[0], g.x[3]);
-    double d12 = dist3(g.x[1], g.x[2]), d13 = dist3(g.x[1], g.x[3]), d23 = dist3(g.x[2], g.x[3]);
-    double a = sel4(p, d23, d23, d13, d12), b = sel4(p, d13, d03, d03, d02), c = sel4(p, d12, d02, d01, d01);
-    double area = 0.25 * sqrt((a + b + c) * (b + c - a) * (c + a - b) * (a + b - c));
-    fd = a * b * c / (4.0 * area);
-  }
-  TetGeom gn;
-  load_tet_geom(in.pts, in.ctet, in.cedge, in.cpar, n, gn);
-  double sgn[9];
-  load_sigma(in, n, sgn);
-#pragma unroll 1
-  for (int s = 0; s < in.nsol; ++s) {
-    double ur[6], ui[6], urn[6], uin[6];
-    load_coef(in, g, s, ur, ui);
-    load_coef(in, gn, s, urn, uin);
-    double cr[3], ci[3], crn[3], cin[3];
-    curl_of(g, ur, ui, cr, ci);
-    curl_of(gn, urn, uin, crn, cin);
-    double dr[3] = {cr[0] - crn[0], cr[1] - crn[1], cr[2] - crn[2]};
-    double di[3] = {ci[0] - cin[0], ci[1] - cin[1], ci[2] - cin[2]};
-    double xr0 = dr[1] * nrm[2] - dr[2] * nrm[1], xr1 = dr[2] * nrm[0] - dr[0] * nrm[2],
-           xr2 = dr[0] * nrm[1] - dr[1] * nrm[0];
-    double xi0 = di[1] * nrm[2] - di[2] * nrm[1], xi1 = di[2] * nrm[0] - di[0] * nrm[2],
-           xi2 = di[0] * nrm[1] - di[1] * nrm[0];
-    const double cross2 = xr0 * xr0 + xr1 * xr1 + xr2 * xr2 + xi0 * xi0 + xi1 * xi1 + xi2 * xi2;
-    double dotj = 0, crossh = 0;
+      for (int d = 0; d < 3; ++d) y[p][d] = make_double2(0, 0);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      // face vertices (p+1, p+2, p+3) mod 4 get 2/3 (rotated by q) or 1/6
-      const int hot = (p + 1 + q) & 3;
-      double lam[4], y[3];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) lam[i] = (i == p) ? 0.0 : ((i == hot) ? 2.0 / 3.0 : 1.0 / 6.0);
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        y[d] = lam[0] * g.x[0][d] + lam[1] * g.x[1][d] + lam[2] * g.x[2][d] + lam[3] * g.x[3][d];
-      double lamn[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) lamn[i] = lambda_at(gn, i, y);
-      double er[3], ei[3], ern[3], ein[3];
-      field_at(g, lam, ur, ui, er, ei);
-      field_at(gn, lamn, urn, uin, ern, ein);
-      double jr = 0, ji = 0;
+    for (int k = 0; k < 6; ++k) {
+      const int p = kEdgeP(k), q = kEdgeQ(k);
+      const double2 u = __ldg(in.sol[s] + g.ge[k]);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        double sr = sg[3 * d] * er[0] + sg[3 * d + 1] * er[1] + sg[3 * d + 2] * er[2];
-        double si = sg[3 * d] * ei[0] + sg[3 * d + 1] * ei[1] + sg[3 * d + 2] * ei[2];
-        double snr = sgn[3 * d] * ern[0] + sgn[3 * d + 1] * ern[1] + sgn[3 * d + 2] * ern[2];
-        double sni = sgn[3 * d] * ein[0] + sgn[3 * d + 1] * ein[1] + sgn[3 * d + 2] * ein[2];
-        jr += (sr - snr) * nrm[d];
-        ji += (si - sni) * nrm[d];
+        cmad(y[p][d], g.gr[q][d], u);
+        cmad(y[q][d], -g.gr[p][d], u);
       }
-      dotj += (jr * jr + ji * ji) * jxw_f;
-      crossh += cross2 * jxw_f;
     }
-    double v = (dotj + crossh) * fd / 2.0;
-    fe[((long)s * nt + t) * 4 + f] = v;
-    fe[((long)s * nt + n) * 4 + non] = v;
-  }
-}
-
-// eta[s][t] = vol + fe[0] + fe[1] + fe[2] + fe[3] (the reference's order), then
-// the primal x dual combination sqrt(eta_p * eta_d) (src/em_fwd.cc:1172-1177).
-__global__ void estimate_sum_kernel(int nt, int nsol, const double *__restrict__ vol, const double *__restrict__ fe,
-                                    double *__restrict__ eta) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)nt * nsol) return;
-  double v = vol[i];
 #pragma unroll
-  for (int f = 0; f < 4; ++f) v += fe[i * 4 + f];
-  eta[i] = v;
+    for (int p = 0; p < 4; ++p) {
+      double2 z[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        z[d] = make_double2(0, 0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cmad(z[d], sg[3 * d + c], y[p][c]);
+        sum[d].x += z[d].x;
+        sum[d].y += z[d].y;
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) y[p][d] = z[d];
+    }
+    double v = 0;
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double re = fma(A - B, y[p][d].x, B * sum[d].x), im = fma(A - B, y[p][d].y, B * sum[d].y);
+        v += re * re + im * im;
+      }
+    v *= w;
+    const long o = ((long)s * nt + t) * 4;
+    if (nb.x >= 0) v += fe[o];
+    if (nb.y >= 0) v += fe[o + 1];
+    if (nb.z >= 0) v += fe[o + 2];
+    if (nb.w >= 0) v += fe[o + 3];
+    eta[(long)s * nt + t] = v;
+    es[s] = v;
+  }
+  if (!err) return;
+  const double dual = in.nsol == 3 ? es[2] : es[1];
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+    if (s < in.nsol - 1) err[(long)s * nt + t] = sqrt(es[s] * dual);
 }
 
-__global__ void combine_err_kernel(int nt, int nsol, const double *__restrict__ eta, double *__restrict__ err) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const double *dual = eta + (long)(nsol - 1) * nt;
-  for (int s = 0; s < nsol - 1; ++s) err[(long)s * nt + t] = sqrt(eta[(long)s * nt + t] * dual[t]);
+// interior faces from the lower tet's side, for estimate_face_kernel
+void build_faces(Context &c) {
+  std::vector<int> f;
+  f.reserve(2 * (size_t)c.nt);
+  for (int t = 0; t < c.nt; ++t)
+    for (int k = 0; k < 4; ++k)
+      if (c.h_nbr[4 * (size_t)t + k] > t) f.push_back(4 * t + k);
+  c.n_faces = (int)f.size();
+  c.faces.upload(f, c.stream);
+  EMG_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 void launch_estimate(Context &c, double omega, int nsol, const double *const *sol_dev, double *eta_dev,
-                     double *err_dev, double *scratch_vol, double *scratch_fe) {
+                     double *err_dev, double *scratch_fe) {
   EstIn in;
   in.pts = c.pts.p;
   in.ctet = c.ctet.p;
@@ -261,17 +310,13 @@ void launch_estimate(Context &c, double omega, int nsol, const double *const *so
   in.nsol = nsol;
   for (int s = 0; s < 3; ++s) in.sol[s] = s < nsol ? (const double2 *)sol_dev[s] : nullptr;
   in.omega = omega;
-  estimate_cell_kernel<<<(unsigned)((c.nt + 127) / 128), 128, 0, c.stream>>>(in, c.nt, scratch_vol);
-  EMG_LAUNCH_CHECK();
-  estimate_face_kernel<<<(unsigned)(((long)c.nt * 4 + 127) / 128), 128, 0, c.stream>>>(in, c.nt, scratch_fe);
-  EMG_LAUNCH_CHECK();
-  long n = (long)c.nt * nsol;
-  estimate_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c.stream>>>(c.nt, nsol, scratch_vol, scratch_fe, eta_dev);
-  EMG_LAUNCH_CHECK();
-  if (err_dev) {
-    combine_err_kernel<<<(unsigned)((c.nt + 255) / 256), 256, 0, c.stream>>>(c.nt, nsol, eta_dev, err_dev);
+  if (c.n_faces > 0) {
+    estimate_face_kernel<<<(unsigned)((c.n_faces + 127) / 128), 128, 0, c.stream>>>(in, c.nt, c.n_faces, c.faces.p,
+                                                                                    scratch_fe);
     EMG_LAUNCH_CHECK();
   }
+  estimate_cell_kernel<<<(unsigned)((c.nt + 127) / 128), 128, 0, c.stream>>>(in, c.nt, scratch_fe, eta_dev, err_dev);
+  EMG_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------------
@@ -380,9 +425,9 @@ namespace {
 constexpr int kNoAllocMaxTets = 131072;  // largest mesh the fixed scratch serves
 constexpr int kNoAllocMaxSol = 3;        // MT: XY, YX and the dual solution
 
-// volume terms (n_sol x T) followed by face terms (n_sol x T x 4): 15.7 MB,
-// held on every GPU that loads the library until the process exits
-__device__ __align__(256) double g_estimate_scratch[kNoAllocMaxSol * kNoAllocMaxTets * 5];
+// face terms (n_sol x T x 4): 12.6 MB, held on every GPU that loads the library
+// until the process exits
+__device__ __align__(256) double g_estimate_scratch[kNoAllocMaxSol * kNoAllocMaxTets * 4];
 
 }  // namespace
 
@@ -428,9 +473,9 @@ extern "C" int emg_estimate_error_noalloc(emg_context *ctx, int fidx, int tidx, 
     }
     check_cuda(cudaSetDevice(c.device), "cudaSetDevice", __FILE__, __LINE__);
     double *scratch = noalloc_scratch_address(c.device);
-    // every volume and face entry is written before it is read, so nothing
-    // left in the array by an earlier call needs clearing
-    launch_estimate(c, 2 * PI * c.freqs[fidx], nsol, sp, eta_dev, err_dev, scratch, scratch + (size_t)nsol * c.nt);
+    // every face entry is written before it is read, so nothing left in the
+    // array by an earlier call needs clearing
+    launch_estimate(c, 2 * PI * c.freqs[fidx], nsol, sp, eta_dev, err_dev, scratch);
     check_cuda(cudaStreamSynchronize(c.stream), "cudaStreamSynchronize", __FILE__, __LINE__);
   } catch (const Error &e) {
     set_last_error(e.what());

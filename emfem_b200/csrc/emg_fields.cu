@@ -19,6 +19,7 @@
 #include <array>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <vector>
 
 #include "emg_api.h"
@@ -149,21 +150,25 @@ int emg_interpolate_fields_block_dev(emg_context *c, int k, const double *freqs,
   if (n == 0) return EMG_OK;
   for (int r = 0; r < n; ++r)
     if (tets[r] < 0 || tets[r] >= c->nt) fail(EMG_ERR_USER, "Receiver %d is not found in mesh.", r);
-  std::vector<double> om(k);
+  // receivers, frequencies and cells go up in one copy, into one buffer that
+  // also takes the result
+  const size_t nin = (size_t)n * 3 + k + ((size_t)n + 1) / 2;
+  std::vector<double> in(nin);
+  std::copy(pts, pts + 3 * (size_t)n, in.begin());
   for (int j = 0; j < k; ++j) {
     need(freqs[j] > 0, EMG_ERR_ARG, "frequencies must be positive");
-    om[j] = 2 * PI * freqs[j];
+    in[3 * (size_t)n + j] = 2 * PI * freqs[j];
   }
-  DBuf<double> drx, dom, deh((size_t)n * k * 12);
-  DBuf<int> dt;
-  drx.upload(pts, (size_t)n * 3, c->stream);
-  dt.upload(tets, (size_t)n, c->stream);
-  dom.upload(om, c->stream);
-  FieldArgs a{c->pts.p, c->ctet.p, c->cedge.p, c->cpar.p, drx.p, dt.p, dom.p, (const double2 *)x_dev, deh.p, n, k};
+  std::memcpy(in.data() + 3 * (size_t)n + k, tets, sizeof(int) * (size_t)n);
+  DBuf<double> buf(nin + (size_t)n * k * 12);
+  EMG_CUDA(cudaMemcpyAsync(buf.p, in.data(), sizeof(double) * nin, cudaMemcpyHostToDevice, c->stream));
+  double *deh = buf.p + nin;
+  FieldArgs a{c->pts.p, c->ctet.p, c->cedge.p, c->cpar.p, buf.p, (const int *)(buf.p + 3 * (size_t)n + k),
+              buf.p + 3 * (size_t)n, (const double2 *)x_dev, deh, n, k};
   const long m = (long)n * k;
   fields_block_kernel<<<(unsigned)((m + 127) / 128), 128, 0, c->stream>>>(a);
   EMG_LAUNCH_CHECK();
-  c->stage.download(eh, deh.p, sizeof(double) * (size_t)n * k * 12, c->stream);
+  c->stage.download(eh, deh, sizeof(double) * (size_t)n * k * 12, c->stream);
   EMG_API_END
 }
 

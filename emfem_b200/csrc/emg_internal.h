@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -165,15 +166,30 @@ struct DBuf {
 // Copies device results to pageable host memory through two pinned buffers: the
 // GPU fills one while the host's threads empty the other.  The driver's own
 // copy to pageable memory goes through one thread (12 MB of error indicators:
-// 1.5 ms).  Returns when host[0 .. bytes) is written.
+// 1.5 ms).  One pair of buffers serves every device context of the process,
+// one copy at a time (pinning them takes milliseconds); the last context gives
+// them back.
 struct PinnedStage {
   static constexpr size_t kBytes = size_t(2) << 20;  // each buffer
   char *buf[2] = {nullptr, nullptr};
-  cudaEvent_t done[2] = {nullptr, nullptr};
-  PinnedStage() = default;
+  std::mutex mu;
+  PinnedStage();
   PinnedStage(const PinnedStage &) = delete;
   PinnedStage &operator=(const PinnedStage &) = delete;
   ~PinnedStage();
+  static std::shared_ptr<PinnedStage> get();
+};
+
+// a context's way through it
+struct StagedCopy {
+  std::shared_ptr<PinnedStage> stage;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  StagedCopy() = default;
+  StagedCopy(const StagedCopy &) = delete;
+  StagedCopy &operator=(const StagedCopy &) = delete;
+  ~StagedCopy();
+  void open();  // buffers and events; the context's device is current
+  // returns when host[0 .. bytes) is written
   void download(void *host, const void *dev, size_t bytes, cudaStream_t s);
 };
 
@@ -286,7 +302,7 @@ struct Workspace;
 // ---------------------------------------------------------------------------
 struct Context {
   DevicePool pool;  // first member: outlives every buffer below
-  PinnedStage stage;
+  StagedCopy stage;
   int device = 0;
   cudaStream_t stream = nullptr;
   Options opt;
@@ -300,6 +316,8 @@ struct Context {
   DBuf<unsigned char> ebdr;
   DBuf<int> ctet, cedge;           // canonical tets: sorted vertices, canonical edges
   DBuf<signed char> cpar;          // parity of the vertex sort
+  DBuf<int> faces;                 // interior faces, 4 t + f of their lower tet
+  int n_faces = 0;
   // model
   int aniso_form = 0;
   std::vector<double> rho;
@@ -375,6 +393,7 @@ void sigma_table(int aniso_form, int nrho, int ncol, const double *rho, std::vec
 void build_sparsity(Context &c);          // host: CSR pattern (make_sparsity_patterns)
 void build_vertex_pattern(Context &c);    // host: vertex adjacency + incidence
 void canonicalize(Context &c);            // device: sorted tets + canonical edges
+void build_faces(Context &c);             // the interior face list (estimator)
 void build_slot_maps(Context &c);         // device: edge incidence records, tet -> vertex CSR slots
 void assemble_edge(Context &c);           // device: C, Ms, bdr cells
 void assemble_nodal(Context &c, HCsr out[4]);  // device + download (G, Pi_x, Pi_y, Pi_z)

@@ -157,7 +157,7 @@ int emg_estimate_error(emg_context *ctx, int fidx, int tidx, double *err, double
  * library allocate device memory during a run (an application whose memory
  * manager owns the device, or code that must not be stalled by
  * cudaMalloc/cudaFree).  No counterpart in the reference.  The scratch lives
- * in a fixed 15.7 MB device array of the library (held on every GPU that
+ * in a fixed 12.6 MB device array of the library (held on every GPU that
  * loads it), so meshes above 131072 tets are rejected with EMG_ERR_ARG.
  * err_dev (n_err x T) and eta_dev (n_sol x T) are caller-owned device
  * buffers laid out as in emg_estimate_error.  The array's device address is

@@ -1,0 +1,60 @@
+"""Row-wise assembly on fans of tets around an axis, against the oracle.
+
+The axis edges of a fan collect a term from every tet around them: 3 and 40
+tets per axis edge stay inside the record's 9-bit positions and the block's
+tile of row slots, 200 tets on 5 consecutive axis edges (601 slots per row)
+exceed both, so that columns are searched for and rows summed in place.
+Bars of the other assembly tests: pattern and boundary cells equal, values to
+1e-12 of the largest.
+"""
+
+import numpy as np
+import pytest
+
+import emfem_b200 as E
+from emfem_b200 import meshgen as mg
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _fan(n_ring, n_axis, shuffle):
+    a = np.linspace(0, 2 * np.pi, n_ring, endpoint=False)
+    ring = np.stack([1.3 * np.cos(a), np.sin(a), 0.45 + 0.02 * np.sin(3 * a)], axis=1)
+    axis = np.stack([np.zeros(n_axis), np.zeros(n_axis), np.linspace(0, 1, n_axis)], axis=1)
+    pts = np.concatenate([ring, axis]) * 100.0
+    tets = [[n_ring + k, n_ring + k + 1, i, (i + 1) % n_ring] for k in range(n_axis - 1) for i in range(n_ring)]
+    tets = np.array(tets, dtype=np.int64)
+    if shuffle:  # vertex ids in another order: every orientation of the record's signs
+        perm = np.random.default_rng(n_ring).permutation(pts.shape[0])
+        inv = np.empty_like(perm)
+        inv[perm] = np.arange(perm.size)
+        pts, tets = pts[perm], inv[tets]
+    tets = mg.orient_positive(pts, tets)
+    attr = (np.arange(tets.shape[0]) % 3).astype(np.int32)
+    return mg.build_topology(pts, tets, attr)
+
+
+@pytest.mark.parametrize("n_ring,n_axis", [(3, 2), (40, 3), (200, 6)])
+@pytest.mark.parametrize("shuffle", [False, True])
+def test_fan_matches_oracle(n_ring, n_axis, shuffle):
+    m = _fan(n_ring, n_axis, shuffle)
+    model = mg.Model(mg.ARBITRARY, np.array([[10.0, 30.0, 5.0, 20.0, -35.0, 50.0], [1.0, 2.0, 4.0, 10.0, 0.0, 5.0],
+                                             [100.0, 100.0, 100.0, 0.0, 0.0, 0.0]]))
+    om = O.Mesh(m)
+    orp, oci = O.sparsity(om)
+    Co, Mo, bo = O.assemble(om, model, 2.0, orp, oci)
+    with E.EMContext(0) as c:
+        c.set_mesh(m)
+        c.set_model(model)
+        c.set_frequencies([2.0])
+        c.create_linear_system(0)
+        c.assemble_matrix(0)
+        rp, ci = c.make_sparsity_patterns()
+        C, M, bdr = c.get_matrices()
+        c.assemble_matrix(0)
+        C2, M2, _ = c.get_matrices()
+    assert np.array_equal(rp, orp) and np.array_equal(ci, oci) and np.array_equal(bdr, bo)
+    assert np.abs(C - Co).max() <= 1e-12 * np.abs(Co).max()
+    assert np.abs(M - Mo).max() <= 1e-12 * max(np.abs(Mo).max(), 1e-300)
+    assert np.array_equal(C, C2) and np.array_equal(M, M2)  # a fixed summation order
