@@ -21,7 +21,7 @@ constexpr bool spmm_legal() {
   return (K % V) == 0 && (K / V) * NL <= 32 && (32 % ((K / V) * NL)) == 0 && sizeof(T) * V <= 16;
 }
 
-template <typename T, int K, int V, int NL, bool PK = false, int MINB = 1>
+template <typename T, int K, int V, int NL, bool PK = false, int MINB = 1, int U = 4, bool LATE = false>
 void spmm_launch(const SpmmArgs &a, cudaStream_t s) {
   constexpr int G = NL * (K / V);
   constexpr int RPW = 32 / G;
@@ -29,7 +29,7 @@ void spmm_launch(const SpmmArgs &a, cudaStream_t s) {
   long threads = warps * 32;
   unsigned grid = (unsigned)((threads + 255) / 256);
   if (grid == 0) return;
-  launch_chain(&spmm_kernel<T, K, V, NL, PK, MINB>, grid, 256, s, a.chained, a);
+  launch_chain(&spmm_kernel<T, K, V, NL, PK, MINB, U, LATE>, grid, 256, s, a.chained, a);
 }
 
 // register-capped row-split kernel (nl = 400 + NL packed records, 500 + NL
@@ -39,6 +39,15 @@ template <typename T, int K, int V, int NL, bool PK>
 SpmmFn spmm_pick_capped() {
   if constexpr (spmm_legal<T, K, V, NL>() && (sizeof(T) == 4 || !PK) && K >= 16)
     return &spmm_launch<T, K, V, NL, PK, 4>;
+  else return nullptr;
+}
+
+// nl = 800 + NL: 6 blocks per SM, 2 nonzeros per round, late epilogue loads;
+// whole 16-byte vectors only
+template <typename T, int K, int V, int NL>
+SpmmFn spmm_pick_dense() {
+  if constexpr (spmm_legal<T, K, V, NL>() && sizeof(T) * V == 16 && K >= 8)
+    return &spmm_launch<T, K, V, NL, false, 6, 2, true>;
   else return nullptr;
 }
 
@@ -121,6 +130,8 @@ SpmmFn spmm_pick_nl(int nl) {
   case 104: return spmm_pick_packed<T, K, V, 4>();
   case 601: return spmm_chunk_pick<T, K, V, 1>();
   case 604: return spmm_chunk_pick<T, K, V, 4>();
+  case 801: return spmm_pick_dense<T, K, V, 1>();
+  case 802: return spmm_pick_dense<T, K, V, 2>();
   case 401: return spmm_pick_capped<T, K, V, 1, true>();
   case 402: return spmm_pick_capped<T, K, V, 2, true>();
   case 501: return spmm_pick_capped<T, K, V, 1, false>();
@@ -174,7 +185,8 @@ std::string SpmmTuner::report() const {
        << (std::get<3>(kv.first) & 1 ? " (packed records available)" : "")
        << (std::get<3>(kv.first) & 2 ? " (chunks available)" : "")
        << (kv.second.second < 0 ? " rows kernel B="
-                                : (kv.second.second > 600   ? " chunked, min blocks/SM "
+                                : (kv.second.second > 800   ? " 6 blocks/SM NL="
+                                   : kv.second.second > 600 ? " chunked, min blocks/SM "
                                    : kv.second.second > 500 ? " register-capped NL="
                                    : kv.second.second > 400 ? " packed register-capped NL="
                                    : kv.second.second > 300 ? " packed pipelined U="
@@ -190,8 +202,14 @@ static int row_bucket(const SpmmArgs &a, long nnz) {
   return avg < 6 ? 0 : (avg < 12 ? 1 : (avg < 24 ? 2 : 3));
 }
 
-// row-count class: the edge matrix and the finest nodal levels tune apart
-static int size_class(const SpmmArgs &a) { return a.n >= 1000000 ? 2 : (a.n >= 100000 ? 1 : 0); }
+// row-count class, a factor of two wide: the layout that is fastest at 29000 rows
+// of 21 nonzeros (11.9 us, one lane per row) takes 9.0 us at 11000 of 25,
+// where two lanes take 7.5
+static int size_class(const SpmmArgs &a) {
+  int c = 0;
+  while ((a.n >> c) > 1) ++c;
+  return c;
+}
 
 // Layout of an operator whose rows x column lanes leave most of the chip idle
 // (a quarter of its threads): the widest vectors, and as many lanes per row
@@ -242,9 +260,9 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
       // then ran 17% slower over the solver's mix of smoothing modes.
       std::vector<std::pair<int, int>> cand;
       for (int v : {1, 2, 4})
-        for (int nl : {1, 2, 4, 8, 16, 32, -4, -8, 101, 102, 104, 401, 402, 501, 502, 601, 604}) {
+        for (int nl : {1, 2, 4, 8, 16, 32, -4, -8, 101, 102, 104, 401, 402, 501, 502, 601, 604, 801, 802}) {
           if (((nl > 100 && nl < 200) || (nl > 400 && nl < 500)) && !packed) continue;
-          if (nl > 600 && !chunked) continue;
+          if (nl > 600 && nl < 700 && !chunked) continue;
           if (spmm_fn<T>(K, v, nl)) cand.push_back({v, nl});
         }
       // two interleaved passes, each candidate's best: one slow sample (a
@@ -342,7 +360,7 @@ bool spmm_layout(int K, int v, int nl, const SpmmArgs &a, cudaStream_t s) {
   if (!f) return false;
   const bool packed_variant = (nl > 100 && nl < 200) || (nl > 300 && nl < 400) || (nl > 400 && nl < 500);
   if (packed_variant && (a.pk == nullptr || a.vm == nullptr)) return false;
-  if (nl > 600 && (a.ch == nullptr || a.crp == nullptr || a.vm == nullptr)) return false;
+  if (nl > 600 && nl < 700 && (a.ch == nullptr || a.crp == nullptr || a.vm == nullptr)) return false;
   if (a.n > 0) f(a, s);
   EMG_LAUNCH_CHECK();
   return true;

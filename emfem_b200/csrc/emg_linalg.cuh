@@ -241,8 +241,14 @@ __device__ __forceinline__ void spmm_epilogue(const SpmmArgs &a, int row, int cb
 }
 
 // MINB > 1 caps the registers so that MINB blocks of 256 threads fit on an SM
-// (more warps in flight for the load-latency-bound gathers, a few spills)
-template <typename T, int K, int V, int NL, bool PK = false, int MINB = 1>
+// (more warps in flight for the load-latency-bound gathers, a few spills).
+// LATE reads the row vectors of the epilogue after the row product instead of
+// before it: 12 registers less, so that with U = 2 nonzeros per round 6 blocks
+// fit instead of 4; the other warps hide what the row then waits for.
+// Edge operator, 150k rows, 32 columns, residual / middle / last smoothing
+// step: 39 / 48.7 / 46.4 us (U = 4, 4 blocks) -> 37.2 / 45.0 / 40.7; U = 2 with
+// 5 blocks 40 / 49 / 44, 8 blocks 49 / 57 / 55, U = 4 with 6 blocks 59 / 65 / 62.
+template <typename T, int K, int V, int NL, bool PK = false, int MINB = 1, int U = 4, bool LATE = false>
 __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   constexpr int CL = K / V;
   constexpr int G = NL * CL;
@@ -274,7 +280,6 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   // U nonzeros per lane per round: all index/value loads of the round are
   // issued before the dependent x gathers, so U gathers are in flight at
   // once (rows are short, ~16 nonzeros, and split NL ways)
-  constexpr int U = 4;
   int k0 = kb + sl;
   int j[U];
   T c[U], m[U];
@@ -299,9 +304,9 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
   // the first round of the matrix before the wait: on the small levels that
   // is the whole row, and only the gathers remain of the dependent chain
   fetch();
-  if (valid && sl == 0) epi_diag<T, V>(a, row, two, epi);
+  if (!LATE && valid && sl == 0) epi_diag<T, V>(a, row, two, epi);
   pdl_wait();
-  if (valid && sl == 0) epi_load<T, K, V>(a, row, cb, epi);
+  if (!LATE && valid && sl == 0) epi_load<T, K, V>(a, row, cb, epi);
   while (k0 < ke) {
     T xv[U][V];
 #pragma unroll
@@ -324,6 +329,10 @@ __global__ void __launch_bounds__(256, MINB) spmm_kernel(SpmmArgs a) {
 #pragma unroll
     for (int i = 0; i < V; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
   if (!valid || sl != 0) return;
+  if (LATE) {
+    epi_diag<T, V>(a, row, two, epi);
+    epi_load<T, K, V>(a, row, cb, epi);
+  }
   epi_store<T, K, V>(a, row, cb, acc, w, two, epi);
 }
 

@@ -399,7 +399,8 @@ int emg_spmv_complex_dev(emg_context *ctx, int k, const double *omegas_host, con
  * software-pipelined kernel with chunks of U nonzeros, 400 + NL / 500 + NL
  * the row-split kernel capped at 64 registers (4 blocks per SM; packed
  * records / arrays, fp32, K >= 16), 601 / 604 the chunked kernel (rows in
- * whole chunks of 4 nonzeros; fp32, K >= 8; 604 register-capped).
+ * whole chunks of 4 nonzeros; fp32, K >= 8; 604 register-capped), 800 + NL the
+ * row-split kernel at 6 blocks per SM (K >= 8, whole 16-byte vectors).
  * EMG_ERR_ARG for a layout not built for K.  Tests every kernel the
  * autotuner can pick. */
 int emg_spmm_layout_dev(emg_context *ctx, int fp32, int K, int v, int variant, const double *omegas_host,

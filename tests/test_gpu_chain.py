@@ -64,3 +64,39 @@ def test_block_widths(system, fp32, k, options):
     assert all(i.reason == 0 for i in infos)
     err = np.abs(x - exact[:, cols]).max(axis=0) / np.abs(exact[:, cols]).max(axis=0)
     assert err.max() <= 1e-6, err
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("K", [8, 16, 32, 64])
+@pytest.mark.parametrize("variant", [801, 802])
+def test_dense_residency_layout(system, fp32, K, variant):
+    """y = b - (C + w Ms) x with the 6-blocks-per-SM layout against float64: rows
+    of 9 to 40 nonzeros leave every remainder of its rounds of 2 (and of 2
+    lanes).  Tolerances as in test_gpu_spmm_layouts.py."""
+    import scipy.sparse as sp
+    import torch
+    c = system[0]
+    c.assemble_matrix(0)
+    rp, ci = c.make_sparsity_patterns()
+    Cv, Mv, _ = c.get_matrices()
+    n = rp.size - 1
+    Cm, Mm = sp.csr_matrix((Cv, ci, rp), shape=(n, n)), sp.csr_matrix((Mv / (2 * np.pi * 0.5), ci, rp), shape=(n, n))
+    rng = np.random.default_rng(K)
+    w = 2 * np.pi * np.logspace(-1, 1, K)
+    if K == 16:
+        w = np.repeat(w[::2], 2)  # complex columns: pairs share their frequency
+    dt = torch.float32 if fp32 else torch.float64
+    x = torch.from_numpy(rng.standard_normal((n, K))).to(dt).cuda()
+    b = torch.from_numpy(rng.standard_normal((n, K))).to(dt).cuda()
+    y = torch.full_like(x, float("nan"))
+    torch.cuda.synchronize()
+    v = 4 if fp32 else 2
+    ok = c.spmm_layout_dev(fp32, w, x.data_ptr(), b.data_ptr(), y.data_ptr(), v, variant)
+    assert ok == (K // v * (variant - 800) <= 32)
+    if not ok:
+        return
+    c.synchronize()
+    xh, bh, yh = x.double().cpu().numpy(), b.double().cpu().numpy(), y.double().cpu().numpy()
+    ref = bh - Cm @ xh - (Mm @ xh) * w
+    scale = np.abs(bh) + abs(Cm) @ np.abs(xh) + (abs(Mm) @ np.abs(xh)) * w
+    assert (np.abs(yh - ref) / scale).max() <= (1e-5 if fp32 else 1e-13)
