@@ -2,13 +2,19 @@
 //
 // An iteration is the preconditioner, the operator and four passes over the
 // block vectors: the dots with the previous B-products, the new direction,
-// the two dots of the step length, and the update.  Each reducing pass ends in
-// its last block, which turns the sums into the recurrence scalars of every
-// column and clears them for the next iteration, so there is no scalar
+// the two dots of the step length, and the update.  There is no scalar
 // kernel, memset or copy between the passes (there were 14 launches per
 // iteration around the preconditioner; in a stream each costs the host 3.3 us,
-// more than the GPU needs for it below 20000 rows).  The passes are bandwidth
-// bound above that; a thread handles two columns (16-byte loads).
+// more than the GPU needs for it below 20000 rows): a thread keeps its two
+// columns (16-byte loads) along its grid stride, so the pass that uses a sum
+// forms the scalars of those columns from it, once per thread, and the update
+// ends in its last block, which stores them, retires columns and clears the
+// sums.  With a last block in every reducing pass instead, 64-bit divisions
+// by the row width and 8 blocks per SM (dots / step length, us per pass):
+// 6.1k rows, 16 columns 5.9 / 4.8 -> 1.9 / 1.7, 100k rows, 8 columns 11.5 /
+// 8.5 -> 5.1 / 4.9, 150k rows, 32 columns 39 / 25 -> 14 / 17 (floor of the
+// last: 100 and 115 MB, 15 and 18 us; both partly from L2).  The direction
+// pays 1.8 us for its scalars at the smallest size.
 
 #include <cuda_runtime.h>
 
@@ -25,8 +31,11 @@ namespace {
 
 constexpr int kThreads = 256;
 
-unsigned pass_grid(long pairs) {
-  return (unsigned)std::max(1L, std::min((pairs + kThreads - 1) / kThreads, 148L * 8));
+// blocks of a pass: 4 per SM where every block adds to the same sums and four
+// pairs of a thread are in flight, 8 for the update (4 / 8: dots 14 / 24 us,
+// update pass -9 us at 150k rows and 32 columns)
+unsigned pass_grid(long pairs, int per_sm = 4) {
+  return (unsigned)std::max(1L, std::min((pairs + kThreads - 1) / kThreads, 148L * per_sm));
 }
 
 // out[q * K + c] += the block's sum of v[q][c % 2] over the threads of column
@@ -134,12 +143,14 @@ struct Dirs {
   const double *p[Fcg::kMaxDirs];
 };
 
-// z of the pair i2: stored, or x + G phi formed from the FP32 AMS output
+// z of the pair i2: stored, or x + G phi formed from the FP32 AMS output.  The
+// pairs per row are a power of two and come as its logarithm: the 64-bit
+// division was most of the instructions of the pass
 template <bool SPLIT>
-__device__ __forceinline__ double2 z_at(long i2, int hp, const double2 *z, const Fcg::ZSplit &zs) {
+__device__ __forceinline__ double2 z_at(long i2, int lhp, const double2 *z, const Fcg::ZSplit &zs) {
   if constexpr (!SPLIT) return z[i2];
-  const long e = i2 / hp;
-  const int c2 = (int)(i2 - e * hp);
+  const long e = i2 >> lhp;
+  const int hp = 1 << lhp, c2 = (int)i2 & (hp - 1);
   const int2 v = __ldg(reinterpret_cast<const int2 *>(zs.edges) + e);
   const float2 x = reinterpret_cast<const float2 *>(zs.x)[i2];
   const float2 a = reinterpret_cast<const float2 *>(zs.phi)[(long)v.x * hp + c2];
@@ -147,65 +158,84 @@ __device__ __forceinline__ double2 z_at(long i2, int hp, const double2 *z, const
   return make_double2((double)x.x + ((double)b.x - (double)a.x), (double)x.y + ((double)b.y - (double)a.y));
 }
 
-// dots (z, S_j) of up to 4 directions; the last block of the last group forms
-// beta_j = (z, S_j) / eta_j of all nprev directions (slot[j]: ring slot of j)
+// dots (z, S_j) of the NJ directions from j0 on
 struct Slots {
   int s[Fcg::kMaxDirs];
 };
 
-template <bool SPLIT>
-__global__ void __launch_bounds__(kThreads) fcg_dots_kernel(long pairs, int hp, const double2 *z, Fcg::ZSplit zs,
-                                                            int j0, int nj, Dirs S, double *acc, int nprev, Slots slot,
-                                                            const double *eta, const int *act, double *beta,
-                                                            unsigned *count) {
+template <bool SPLIT, int NJ, int U>
+__global__ void __launch_bounds__(kThreads) fcg_dots_kernel(long pairs, int lhp, const double2 *z, Fcg::ZSplit zs,
+                                                            int j0, Dirs S, double *acc) {
   pdl_trigger();
   pdl_wait();
-  double v[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-  for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < pairs; i += (long)gridDim.x * kThreads) {
-    const double2 zv = z_at<SPLIT>(i, hp, z, zs);
+  double v[NJ][2] = {};
+  const long step = (long)gridDim.x * kThreads;
+  long i = blockIdx.x * (long)kThreads + threadIdx.x;
+  auto add = [&](const double2 &zv, const double2 &sv, int j) {
+    v[j][0] = fma(zv.x, sv.x, v[j][0]);
+    v[j][1] = fma(zv.y, sv.y, v[j][1]);
+  };
+  for (; i + (U - 1) * step < pairs; i += U * step) {  // U pairs in flight
+    double2 zv[U], sv[U][NJ];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (j < nj) {
-        const double2 sv = reinterpret_cast<const double2 *>(S.p[j0 + j])[i];
-        v[j][0] = fma(zv.x, sv.x, v[j][0]);
-        v[j][1] = fma(zv.y, sv.y, v[j][1]);
-      }
+    for (int u = 0; u < U; ++u) {
+      zv[u] = z_at<SPLIT>(i + u * step, lhp, z, zs);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        sv[u][j] = reinterpret_cast<const double2 *>(S.p[j0 + j])[i + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        add(zv[u], sv[u][j], j);
   }
-  const int K = 2 * hp;
-  column_sums<4>(v, nj, hp, acc + j0 * K);
-  if (!last_block(count) || j0 + nj < nprev) return;
-  for (int t = threadIdx.x; t < nprev * K; t += kThreads) {
-    const int j = t / K, c = t - j * K;
-    const double d = take(acc + t), e = eta[slot.s[j] * K + c];
-    beta[t] = (act[c] && e != 0.0) ? d / e : 0.0;
+  for (; i < pairs; i += step) {
+    const double2 zv = z_at<SPLIT>(i, lhp, z, zs);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+      add(zv, reinterpret_cast<const double2 *>(S.p[j0 + j])[i], j);
   }
+  column_sums<NJ>(v, NJ, 1 << lhp, acc + (j0 << (lhp + 1)));
 }
 
-// p = z - sum_j beta_j P_j
-template <bool SPLIT>
-__global__ void __launch_bounds__(kThreads) fcg_direction_kernel(long pairs, int hp, const double2 *z, Fcg::ZSplit zs,
-                                                                 int nprev, Dirs P, const double *beta, double2 *p) {
+// p = z - sum_j beta_j P_j over NJ directions from j0 on, beta_j = (z, S_j) /
+// eta_j of the active columns (slot[j]: ring slot of j; ieta = 1 / eta, for a
+// thread has only one pair)
+template <bool SPLIT, int NJ>
+__global__ void __launch_bounds__(kThreads) fcg_direction_kernel(long pairs, int lhp, const double2 *z,
+                                                                 Fcg::ZSplit zs, int j0, Dirs P, Slots slot,
+                                                                 const double2 *acc, const double2 *ieta,
+                                                                 const int2 *act, double2 *p) {
   pdl_trigger();
   const long i = blockIdx.x * (long)kThreads + threadIdx.x;
+  const int c2 = (int)i & ((1 << lhp) - 1);
   pdl_wait();
   if (i >= pairs) return;
-  const int c = 2 * (int)(i % hp);
-  double2 v = z_at<SPLIT>(i, hp, z, zs);
-  for (int j = 0; j < nprev; ++j) {
-    const double2 pj = reinterpret_cast<const double2 *>(P.p[j])[i];
-    v.x -= beta[2 * j * hp + c] * pj.x;
-    v.y -= beta[2 * j * hp + c + 1] * pj.y;
+  double2 d[NJ + 1], e[NJ + 1], pj[NJ + 1];
+  const int2 on = act[c2];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    d[j] = acc[((j0 + j) << lhp) + c2];
+    e[j] = ieta[(slot.s[j0 + j] << lhp) + c2];
+    pj[j] = reinterpret_cast<const double2 *>(P.p[j0 + j])[i];
+  }
+  double2 v = z_at<SPLIT>(i, lhp, z, zs);
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    v.x -= (on.x ? d[j].x * e[j].x : 0.0) * pj[j].x;
+    v.y -= (on.y ? d[j].y * e[j].y : 0.0) * pj[j].y;
   }
   p[i] = v;
 }
 
-// (p, s), (p, r); the last block: eta = (p, s), alpha = (p, r) / (p, s)
-__global__ void __launch_bounds__(kThreads) fcg_step_kernel(long pairs, int hp, const double2 *p, const double2 *sv,
-                                                            const double2 *r, double *acc, double *eta,
-                                                            const int *act, double *alpha, unsigned *count) {
+// (p, s), (p, r)
+__global__ void __launch_bounds__(kThreads) fcg_step_kernel(long pairs, int lhp, const double2 *p, const double2 *sv,
+                                                            const double2 *r, double *acc) {
   pdl_trigger();
   pdl_wait();
   double v[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll 2
   for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < pairs; i += (long)gridDim.x * kThreads) {
     const double2 a = p[i], b = sv[i], q = r[i];
     v[0][0] = fma(a.x, b.x, v[0][0]);
@@ -213,32 +243,31 @@ __global__ void __launch_bounds__(kThreads) fcg_step_kernel(long pairs, int hp, 
     v[1][0] = fma(a.x, q.x, v[1][0]);
     v[1][1] = fma(a.y, q.y, v[1][1]);
   }
-  const int K = 2 * hp;
-  column_sums<2>(v, 2, hp, acc);
-  if (!last_block(count)) return;
-  for (int c = threadIdx.x; c < K; c += kThreads) {
-    const double ps = take(acc + c), pr = take(acc + K + c);
-    eta[c] = ps;
-    alpha[c] = (act[c] && ps != 0.0) ? pr / ps : 0.0;
-  }
+  column_sums<2>(v, 2, 1 << lhp, acc);
 }
 
-// x += alpha p, r -= alpha s (in every form); the last block counts the
-// iteration of every active column, retires the converged ones (||r_c||^2 <=
-// rtol^2 ||b_c||^2) and flags NaN/Inf: status[0] = active columns left,
-// status[1] = 1 + a non-finite column (0: none)
-__global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int hp, const double *alpha,
-                                                              const double2 *p, const double2 *sv, double *const *xslot,
-                                                              double2 *r, FcgFeed feed, double *acc, double *bn,
+// x += alpha p, r -= alpha s (in every form), alpha = (p, r) / (p, s) of the
+// active columns from their sums.  The last block stores 1 / (p, s) and alpha, counts the iteration of every active column, retires the
+// converged ones (||r_c||^2 <= rtol^2 ||b_c||^2), flags NaN/Inf and clears the
+// sums (acc: the nacc of this iteration's passes, those of the step length at
+// kstep): status[0] = active columns left, status[1] = 1 + a non-finite column
+// (0: none)
+__global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int lhp, const double2 *p,
+                                                              const double2 *sv, double *const *xslot, double2 *r,
+                                                              FcgFeed feed, double *acc, int kstep, int nacc,
+                                                              double *acc_rr, double *ieta, double *alpha, double *bn,
                                                               double rtol2, int *act, int *its, int *status,
                                                               unsigned *count) {
   pdl_trigger();
   pdl_wait();
+  const int hp = 1 << lhp, K = 2 * hp;
   double2 *x = reinterpret_cast<double2 *>(*xslot);
   double v[1][2] = {{0, 0}};
   const long i0 = blockIdx.x * (long)kThreads + threadIdx.x;
-  const int c = 2 * (int)(i0 % hp);  // the stride is a multiple of hp
-  const double a0 = alpha[c], a1 = alpha[c + 1];
+  const int c = 2 * ((int)i0 & (hp - 1));  // the stride is a multiple of hp
+  const double ps0 = acc[kstep + c], ps1 = acc[kstep + c + 1];
+  const double a0 = (act[c] && ps0 != 0.0) ? acc[kstep + K + c] / ps0 : 0.0;
+  const double a1 = (act[c + 1] && ps1 != 0.0) ? acc[kstep + K + c + 1] / ps1 : 0.0;
   for (long i = i0; i < pairs; i += (long)gridDim.x * kThreads) {
     double2 xv = x[i], rv = r[i];
     const double2 pv = p[i], s = sv[i];
@@ -248,17 +277,24 @@ __global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int hp
     rv.y -= a1 * s.y;
     x[i] = xv;
     r[i] = rv;
-    feed_residual(feed, i, i / hp, c, rv);
+    feed_residual(feed, i, i >> lhp, c, rv);
     v[0][0] = fma(rv.x, rv.x, v[0][0]);
     v[0][1] = fma(rv.y, rv.y, v[0][1]);
   }
-  column_sums<1>(v, 1, hp, acc);
+  column_sums<1>(v, 1, hp, acc_rr);
   if (!last_block(count)) return;
   __shared__ int left;
   if (threadIdx.x == 0) left = 0;
+  if (threadIdx.x < hp) {  // blocks start on a row, so this thread's columns are c and c + 1
+    ieta[c] = ps0 != 0.0 ? 1.0 / ps0 : 0.0;
+    ieta[c + 1] = ps1 != 0.0 ? 1.0 / ps1 : 0.0;
+    alpha[c] = a0;
+    alpha[c + 1] = a1;
+  }
   __syncthreads();
-  for (int k = threadIdx.x; k < 2 * hp; k += kThreads) {
-    const double rn = take(acc + k);
+  for (int k = threadIdx.x; k < nacc; k += kThreads) acc[k] = 0.0;
+  for (int k = threadIdx.x; k < K; k += kThreads) {
+    const double rn = take(acc_rr + k);
     if (!act[k]) continue;
     its[k]++;
     if (!isfinite(rn)) {
@@ -272,6 +308,25 @@ __global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int hp
   }
   __syncthreads();
   if (threadIdx.x == 0) status[0] = left;
+}
+
+auto dots_of(bool split, int nj) {
+  switch (nj) {
+  case 1: return split ? &fcg_dots_kernel<true, 1, 4> : &fcg_dots_kernel<false, 1, 4>;
+  case 2: return split ? &fcg_dots_kernel<true, 2, 4> : &fcg_dots_kernel<false, 2, 4>;
+  case 3: return split ? &fcg_dots_kernel<true, 3, 2> : &fcg_dots_kernel<false, 3, 2>;
+  default: return split ? &fcg_dots_kernel<true, 4, 2> : &fcg_dots_kernel<false, 4, 2>;
+  }
+}
+
+auto direction_of(bool split, int nj) {
+  switch (nj) {
+  case 0: return split ? &fcg_direction_kernel<true, 0> : &fcg_direction_kernel<false, 0>;
+  case 1: return split ? &fcg_direction_kernel<true, 1> : &fcg_direction_kernel<false, 1>;
+  case 2: return split ? &fcg_direction_kernel<true, 2> : &fcg_direction_kernel<false, 2>;
+  case 3: return split ? &fcg_direction_kernel<true, 3> : &fcg_direction_kernel<false, 3>;
+  default: return split ? &fcg_direction_kernel<true, 4> : &fcg_direction_kernel<false, 4>;
+  }
 }
 
 }  // namespace
@@ -299,17 +354,19 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
     }
   }
   acc.alloc((size_t)(mmax + 4) * K);
-  eta.alloc((size_t)mmax * K);
+  ieta.alloc((size_t)mmax * K);
   alpha.alloc(K);
-  beta.alloc((size_t)mmax * K);
   bn.alloc(K);
   xslot.alloc(1);
   act.alloc(K);
   itsd.alloc(K);
   status.alloc(2);
-  count.alloc(4);
+  count.alloc(2);
   if (!h_status.p) EMG_CUDA(cudaMallocHost((void **)&h_status.p, 2 * sizeof(int)));
-  double *acc_step = acc.p + (size_t)mmax * K, *acc_rr = acc_step + 2 * K, *acc_bb = acc_rr + K;
+  const int lhp = K == 2 ? 0 : K == 4 ? 1 : K == 8 ? 2 : K == 16 ? 3 : K == 32 ? 4 : 5;
+  const unsigned dir_grid = (unsigned)((pairs + kThreads - 1) / kThreads);
+  const int kstep = mmax * K;  // where the sums of the step length lie
+  double *acc_rr = acc.p + kstep + 2 * K, *acc_bb = acc_rr + K;
   // a solve that failed half way may have left sums behind
   acc.zero(s);
   count.zero(s);
@@ -332,7 +389,7 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
       add(P[j].p);
       add(S[j].p);
     }
-    for (const void *p : {(const void *)acc.p, (const void *)eta.p, (const void *)alpha.p, (const void *)beta.p,
+    for (const void *p : {(const void *)acc.p, (const void *)ieta.p, (const void *)alpha.p,
                           (const void *)bn.p, (const void *)xslot.p, (const void *)act.p, (const void *)itsd.p,
                           (const void *)status.p, (const void *)count.p, (const void *)feed.r32,
                           (const void *)feed.jf.y, (const void *)feed.jf.d, (const void *)feed.jd.y,
@@ -356,25 +413,24 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
       Pd.p[j] = P[sl.s[j]].p;
     }
     for (int j0 = 0; j0 < nprev; j0 += 4) {
-      const int nj = std::min(4, nprev - j0);
-      auto k = zs ? &fcg_dots_kernel<true> : &fcg_dots_kernel<false>;
-      launch_chain(k, pass_grid(pairs), kThreads, s, true, pairs, hp, (const double2 *)z.p, z0, j0, nj, Sd, acc.p, nprev,
-                   sl, eta.p, act.p, beta.p, count.p);
+      launch_chain(dots_of(zs != nullptr, std::min(4, nprev - j0)), pass_grid(pairs), kThreads, s, true, pairs, lhp,
+                   (const double2 *)z.p, z0, j0, Sd, acc.p);
       EMG_LAUNCH_CHECK();
     }
-    auto kd = zs ? &fcg_direction_kernel<true> : &fcg_direction_kernel<false>;
-    launch_chain(kd, (unsigned)((pairs + kThreads - 1) / kThreads), kThreads, s, true, pairs, hp, (const double2 *)z.p,
-                 z0, nprev, Pd, beta.p, (double2 *)P[head].p);
-    EMG_LAUNCH_CHECK();
     double *p = P[head].p, *sv = S[head].p;
+    for (int j0 = 0; j0 == 0 || j0 < nprev; j0 += 4) {  // a later group goes on from p
+      launch_chain(direction_of(zs && j0 == 0, std::min(4, nprev - j0)), dir_grid, kThreads, s, true, pairs, lhp,
+                   (const double2 *)(j0 ? p : z.p), z0, j0, Pd, sl, (const double2 *)acc.p, (const double2 *)ieta.p,
+                   (const int2 *)act.p, (double2 *)p);
+      EMG_LAUNCH_CHECK();
+    }
     opB(p, sv);
-    launch_chain(&fcg_step_kernel, pass_grid(pairs), kThreads, s, true, pairs, hp, (const double2 *)p,
-                 (const double2 *)sv, (const double2 *)r.p, acc_step, eta.p + (size_t)head * K, act.p, alpha.p,
-                 count.p + 1);
+    launch_chain(&fcg_step_kernel, pass_grid(pairs), kThreads, s, true, pairs, lhp, (const double2 *)p,
+                 (const double2 *)sv, (const double2 *)r.p, acc.p + kstep);
     EMG_LAUNCH_CHECK();
-    launch_chain(&fcg_update_kernel, pass_grid(pairs), kThreads, s, true, pairs, hp, alpha.p, (const double2 *)p,
-                 (const double2 *)sv, xslot.p, (double2 *)r.p, feed, acc_rr, bn.p, rtol * rtol, act.p, itsd.p, status.p,
-                 count.p + 2);
+    launch_chain(&fcg_update_kernel, pass_grid(pairs, 8), kThreads, s, true, pairs, lhp, (const double2 *)p,
+                 (const double2 *)sv, xslot.p, (double2 *)r.p, feed, acc.p, kstep, kstep + 2 * K, acc_rr,
+                 ieta.p + (size_t)head * K, alpha.p, bn.p, rtol * rtol, act.p, itsd.p, status.p, count.p + 1);
     EMG_LAUNCH_CHECK();
   };
   auto run = [&](int head, int nprev) {

@@ -19,11 +19,10 @@ from exact_solve import exact_solutions
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def system():
+def build(cells):
     import torch
     freqs = np.array([0.5, 4.0])
-    prob = mg.marine_csem(1200, freqs=freqs, n_tx=3, name="chain")
+    prob = mg.marine_csem(cells, freqs=freqs, n_tx=3, name="chain")
     c = E.EMContext(0)
     c.set_mesh(prob.mesh)
     c.set_model(prob.model)
@@ -43,8 +42,14 @@ def system():
         Cv, Mv, _ = c.get_matrices()
         jobs.append((rp, ci, Cv, Mv, np.conj(s[:, 3 * f:3 * f + 3])))
     exact = np.concatenate(exact_solutions(jobs), axis=1)
-    yield c, colf, s, exact
-    c.close()
+    return c, colf, s, exact
+
+
+@pytest.fixture(scope="module")
+def system():
+    b = build(1200)
+    yield b
+    b[0].close()
 
 
 @pytest.mark.parametrize("fp32", [True, False])
@@ -100,3 +105,38 @@ def test_dense_residency_layout(system, fp32, K, variant):
     ref = bh - Cm @ xh - (Mm @ xh) * w
     scale = np.abs(bh) + abs(Cm) @ np.abs(xh) + (abs(Mm) @ np.abs(xh)) * w
     assert (np.abs(yh - ref) / scale).max() <= (1e-5 if fp32 else 1e-13)
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("mmax", [1, 3, 4, 5, 9])
+def test_fcg_truncations(system, fp32, mmax):
+    """The passes over the FCG directions go in groups of up to four: every
+    group size, a second and a third group."""
+    if fp32 and mmax > 4:
+        pytest.skip("refused with the FP32 preconditioner")
+    c, colf, s, exact = system
+    c.process_options("-emg_amg_max_coarse 40 -emg_restrict_smooth 1 -emg_smoother chebyshev "
+                      f"-emg_block_fcg_mmax {mmax}")
+    c.assemble_matrix(0)
+    x, infos = c.solve_block(colf[:4], s[:, :4], rtol=1e-8, max_it=200, inner_fp32=fp32)
+    c.process_options("-emg_block_fcg_mmax 2")
+    assert all(i.reason == 0 for i in infos)
+    err = np.abs(x - exact[:, :4]).max(axis=0) / np.abs(exact[:, :4]).max(axis=0)
+    assert err.max() <= 1e-6, err
+
+
+@pytest.mark.parametrize("mmax", [2, 3])
+def test_fcg_long_vectors(mmax):
+    """Block vectors longer than four grids of the passes, with a remainder:
+    several pairs of a thread in flight."""
+    c, colf, s, exact = build(16000)
+    try:
+        assert s.shape[0] * 32 > 4 * 4 * 148 * 256
+        cols = np.arange(32) % 6
+        c.process_options(f"-emg_block_fcg_mmax {mmax}")
+        x, infos = c.solve_block(colf[cols], s[:, cols], rtol=1e-8, max_it=200, inner_fp32=True)
+        assert all(i.reason == 0 for i in infos)
+        err = np.abs(x - exact[:, cols]).max(axis=0) / np.abs(exact[:, cols]).max(axis=0)
+        assert err.max() <= 1e-6, err
+    finally:
+        c.close()
