@@ -171,24 +171,13 @@ __device__ __forceinline__ int find_col(const int *__restrict__ ci, int b, int e
   return lo;
 }
 
-// Record of an (edge, tet) incidence for assemble_edge_kernel.  The tet's
-// vertices are taken in the order (a, b, c, d): a < b the edge's end points,
-// c < d the other two; its edges in the order ab, ac, ad, bc, bd, cd.
-//   einc[j]: the tet, with its canonical edge index k in bits 28..30
-//   erec[j]: 9 bits per edge: its position in the row (511: search for it),
-//            bits 54..57: whether c < a, d < a, c < b, d < b (the edge then
-//            runs against its global orientation), bits 58..63: whether each
-//            edge is on the boundary
+// Record of an (edge, tet) incidence for assemble_edge_kernel:
+//   einc[j]: the tet, with the edge's canonical index k in bits 28..30
+//   erec[j]: per canonical edge l of the tet 9 bits, its position in the
+//            row (511: search for it), and in bit 58 + l whether it is on the
+//            boundary
 constexpr int kTetBits = 28;
 constexpr unsigned kSearch = 511;
-
-// positions (in the sorted tet) of the vertices a, b, c, d for edge k
-__host__ __device__ constexpr int kOther(int k, int which) {
-  return which == 0 ? (kEdgeP(k) == 0 ? (kEdgeQ(k) == 1 ? 2 : 1) : 0)
-                    : (kEdgeQ(k) == 3 ? (kEdgeP(k) == 2 ? 1 : 2) : 3);
-}
-// canonical edge joining sorted positions i < j
-__host__ __device__ constexpr int kEdgeOf(int i, int j) { return i == 0 ? j - 1 : (i == 1 ? j + 1 : 5); }
 
 __global__ void edge_records_kernel(int ne, const int *__restrict__ inc_rp, int *__restrict__ inc,
                                     const int *__restrict__ cedge, const unsigned char *__restrict__ ebdr,
@@ -199,25 +188,15 @@ __global__ void edge_records_kernel(int ne, const int *__restrict__ inc_rp, int 
   const int kb = __ldg(rp + e), ke = __ldg(rp + e + 1);
   for (int j = __ldg(inc_rp + e); j < __ldg(inc_rp + e + 1); ++j) {
     const int t = inc[j];
-    int ge[6], k = 0;
-    for (int l = 0; l < 6; ++l) {
-      ge[l] = __ldg(cedge + 6 * (long)t + l);
-      if (ge[l] == e) k = l;
-    }
-    const int v[4] = {kEdgeP(k), kEdgeQ(k), kOther(k, 0), kOther(k, 1)};
     unsigned long long r = 0;
-    int q = 0;
-    for (int x = 0; x < 4; ++x)
-      for (int y = x + 1; y < 4; ++y, ++q) {
-        const int lo = min(v[x], v[y]), hi = max(v[x], v[y]), g = ge[kEdgeOf(lo, hi)];
-        const int pos = find_col(ci, kb, ke, g) - kb;
-        r |= (unsigned long long)(pos < (int)kSearch ? (unsigned)pos : kSearch) << (9 * q);
-        if (__ldg(ebdr + g)) r |= 1ull << (58 + q);
-      }
-    if (v[2] < v[0]) r |= 1ull << 54;
-    if (v[3] < v[0]) r |= 1ull << 55;
-    if (v[2] < v[1]) r |= 1ull << 56;
-    if (v[3] < v[1]) r |= 1ull << 57;
+    int k = 0;
+    for (int l = 0; l < 6; ++l) {
+      const int g = __ldg(cedge + 6 * (long)t + l);
+      if (g == e) k = l;
+      const int pos = find_col(ci, kb, ke, g) - kb;
+      r |= (unsigned long long)(pos < (int)kSearch ? (unsigned)pos : kSearch) << (9 * l);
+      if (__ldg(ebdr + g)) r |= 1ull << (58 + l);
+    }
     rec[j] = r;
     inc[j] = t | (k << kTetBits);
   }
@@ -311,12 +290,6 @@ void canonicalize(Context &c) {
   if (hb) fail(EMG_ERR_USER, "tet %d: tet2edgelist does not match tetrahedronlist/edgelist", hb - 1);
 }
 
-__device__ __forceinline__ void cross3(const double *a, const double *b, double *o) {
-  o[0] = a[1] * b[2] - a[2] * b[1];
-  o[1] = a[2] * b[0] - a[0] * b[2];
-  o[2] = a[0] * b[1] - a[1] * b[0];
-}
-
 struct ElemIn {
   const double *pts;
   const int *ctet, *cedge, *attr;
@@ -324,6 +297,33 @@ struct ElemIn {
   const unsigned char *ebdr;
   const double *sig;
 };
+
+// S_ab = grad l_a . sigma grad l_b (packed, a <= b)
+__device__ __forceinline__ void grad_products(const ElemIn &in, int t, const TetGeom &g, double S[10]) {
+  const double *sg = in.sig + 9 * (long)__ldg(in.attr + t);
+  double s[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s[k] = __ldg(sg + k);
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int q = p; q < 4; ++q) {
+      double sq0 = s[0] * g.gr[q][0] + s[1] * g.gr[q][1] + s[2] * g.gr[q][2];
+      double sq1 = s[3] * g.gr[q][0] + s[4] * g.gr[q][1] + s[5] * g.gr[q][2];
+      double sq2 = s[6] * g.gr[q][0] + s[7] * g.gr[q][1] + s[8] * g.gr[q][2];
+      S[sym_idx(p, q)] = g.gr[p][0] * sq0 + g.gr[p][1] * sq1 + g.gr[p][2] * sq2;
+    }
+}
+
+// curl of the edge function l_a grad l_b - l_b grad l_a; the roundings are
+// spelled out because an edge must give the same number as a row and as a column
+__device__ __forceinline__ void edge_curl(const double ga[3], const double gb[3], double cu[3]) {
+  cu[0] = 2.0 * fma(ga[1], gb[2], -__dmul_rn(ga[2], gb[1]));
+  cu[1] = 2.0 * fma(ga[2], gb[0], -__dmul_rn(ga[0], gb[2]));
+  cu[2] = 2.0 * fma(ga[0], gb[1], -__dmul_rn(ga[1], gb[0]));
+}
+
+__device__ __forceinline__ double pick3(int i, double a, double b, double c) { return i == 0 ? a : (i == 1 ? b : c); }
 
 // Element matrices of tet t in canonical order: c (curl-curl / mu) and ms
 // (mass without omega), boundary rows/columns zeroed as
@@ -334,28 +334,11 @@ struct ElemIn {
 __device__ __forceinline__ bool element_matrices(const ElemIn &in, int t, double c[36], double ms[36],
                                                  TetGeom &g) {
   load_tet_geom(in.pts, in.ctet, in.cedge, in.cpar, t, g);
-  const double *sg = in.sig + 9 * (long)__ldg(in.attr + t);
-  double s[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) s[k] = __ldg(sg + k);
   double S[10];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = p; q < 4; ++q) {
-      double sq0 = s[0] * g.gr[q][0] + s[1] * g.gr[q][1] + s[2] * g.gr[q][2];
-      double sq1 = s[3] * g.gr[q][0] + s[4] * g.gr[q][1] + s[5] * g.gr[q][2];
-      double sq2 = s[6] * g.gr[q][0] + s[7] * g.gr[q][1] + s[8] * g.gr[q][2];
-      S[sym_idx(p, q)] = g.gr[p][0] * sq0 + g.gr[p][1] * sq1 + g.gr[p][2] * sq2;
-    }
+  grad_products(in, t, g, S);
   double cu[6][3];
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const int a = kEdgeP(k), b = kEdgeQ(k);
-    cu[k][0] = 2.0 * (g.gr[a][1] * g.gr[b][2] - g.gr[a][2] * g.gr[b][1]);
-    cu[k][1] = 2.0 * (g.gr[a][2] * g.gr[b][0] - g.gr[a][0] * g.gr[b][2]);
-    cu[k][2] = 2.0 * (g.gr[a][0] * g.gr[b][1] - g.gr[a][1] * g.gr[b][0]);
-  }
+  for (int k = 0; k < 6; ++k) edge_curl(g.gr[kEdgeP(k)], g.gr[kEdgeQ(k)], cu[k]);
   const double vc = g.vol / MU, vm = g.vol / 20.0;
   bool bd[6];
   bool any = false;
@@ -393,9 +376,15 @@ __device__ __forceinline__ bool element_matrices(const ElemIn &in, int t, double
 // was bound by them.  The row-wise sum recomputes a tet's geometry for each of
 // its six edges instead, needs no atomics, no cleared arrays and no 36-entry
 // slot map per tet, and always sums in the same order.
-// Bound: the data pipe of L1 (85 %: the gathers of a tet's data, each a pass
-// per lane, and the tile's read-modify-writes; C and Ms of a slot lie together
-// for those).  600k tets: 324 us scattered, 211 with separate tiles, 196 now.
+// Every row evaluates its entries as element_matrices does, from the sorted
+// vertices and with the higher edge's operands first: entry (e, f) is the same
+// number as (f, e), and the operator the one that the nodal spaces and G^T B
+// are built from.  (In the air w sigma Ms is 1e-10 of C: rows that each
+// started from their own edge moved solutions by 4e-10.)
+// Bound: the data pipe of L1 (the gathers of a tet's data, each a pass per
+// lane, and the tile's read-modify-writes; C and Ms of a slot lie together for
+// those).  600k tets: 320 us scattered, 206 now; rows that differed from their
+// mirror took 193, 6 blocks per SM instead of 5 (8 bytes spilled) 205.
 constexpr int ASM_ROWS = 128;
 constexpr int ASM_SLOTS = ASM_ROWS * 18;  // a tile holds rows of 18 slots on average (36.9 KB)
 
@@ -419,77 +408,44 @@ __global__ void __launch_bounds__(ASM_ROWS) assemble_edge_kernel(ElemIn in, int 
     for (int j = __ldg(inc_rp + e); j < j1; ++j) {
       const int tk = __ldg(inc + j), t = tk & ((1 << kTetBits) - 1), k = tk >> kTetBits;
       const unsigned long long rc6 = __ldg(rec + j);
-      const int4 vs = __ldg(reinterpret_cast<const int4 *>(in.ctet) + t);
-      const int p = kEdgeP(k), q = kEdgeQ(k), u = kOther(k, 0), w = kOther(k, 1);
-      auto at = [&](int i) { return i == 0 ? vs.x : (i == 1 ? vs.y : (i == 2 ? vs.z : vs.w)); };
-      const int v[4] = {at(p), at(q), at(u), at(w)};
-      double x[4][3];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) x[i][d] = __ldg(in.pts + 3 * (long)v[i] + d);
-      double e1[3], e2[3], e3[3];
+      const int p = kEdgeP(k), q = kEdgeQ(k);
+      TetGeom g;
+      load_tet_geom(in.pts, in.ctet, in.cedge, in.cpar, t, g);
+      double gp[3], gq[3], cu[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        e1[d] = x[1][d] - x[0][d];
-        e2[d] = x[2][d] - x[0][d];
-        e3[d] = x[3][d] - x[0][d];
+        gp[d] = pick3(p, g.gr[0][d], g.gr[1][d], g.gr[2][d]);
+        gq[d] = pick3(q - 1, g.gr[1][d], g.gr[2][d], g.gr[3][d]);
       }
-      double g[4][3];
-      cross3(e2, e3, g[1]);
-      cross3(e3, e1, g[2]);
-      cross3(e1, e2, g[3]);
-      const double det = e1[0] * g[1][0] + e1[1] * g[1][1] + e1[2] * g[1][2];
-      const double inv = 1.0 / det;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        g[1][d] *= inv;
-        g[2][d] *= inv;
-        g[3][d] *= inv;
-        g[0][d] = -(g[1][d] + g[2][d] + g[3][d]);
-      }
-      // (a, b, c, d) is an odd permutation of the sorted vertices for the edges 1 and 4
-      const double par = (double)__ldg(in.cpar + t) * ((k == 1 || k == 4) ? -1.0 : 1.0);
-      const double vol = par * det / 6.0;
-      const double *sg = in.sig + 9 * (long)__ldg(in.attr + t);
-      double S0[4], S1[4];  // grad l_a . sigma grad l_i and grad l_b . sigma grad l_i
+      edge_curl(gp, gq, cu);
+      double Sp[4], Sq[4];  // S_px and S_qx
       {
-        double a0[3], a1[3];  // sigma is symmetric
+        double S[10];
+        grad_products(in, t, g, S);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          a0[d] = __ldg(sg + d) * g[0][0] + __ldg(sg + 3 + d) * g[0][1] + __ldg(sg + 6 + d) * g[0][2];
-          a1[d] = __ldg(sg + d) * g[1][0] + __ldg(sg + 3 + d) * g[1][1] + __ldg(sg + 6 + d) * g[1][2];
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          S0[i] = a0[0] * g[i][0] + a0[1] * g[i][1] + a0[2] * g[i][2];
-          S1[i] = a1[0] * g[i][0] + a1[1] * g[i][1] + a1[2] * g[i][2];
+        for (int x = 0; x < 4; ++x) {
+          Sp[x] = pick3(p, S[sym_idx(0, x)], S[sym_idx(1, x)], S[sym_idx(2, x)]);
+          Sq[x] = pick3(q - 1, S[sym_idx(1, x)], S[sym_idx(2, x)], S[sym_idx(3, x)]);
         }
       }
-      double cu[3];
-      cross3(g[0], g[1], cu);
-      const double vc = 4.0 * vol / MU, vm = vol / 20.0;
-      const bool row_bdr = (rc6 >> 58) & 1;
+      const double vc = g.vol / MU, vm = g.vol / 20.0;
+      const bool row_bdr = (rc6 >> (58 + k)) & 1;
 #pragma unroll
       for (int l = 0; l < 6; ++l) {
-        const int r = l < 3 ? 0 : (l < 5 ? 1 : 2), s = l < 3 ? l + 1 : (l < 5 ? l - 1 : 3);
-        const bool cut = l > 0 && (row_bdr || ((rc6 >> (58 + l)) & 1));
+        const int r = kEdgeP(l), u = kEdgeQ(l);
         double cr[3];
-        cross3(g[r], g[s], cr);
+        edge_curl(g.gr[r], g.gr[u], cr);
         double ckl = vc * (cu[0] * cr[0] + cu[1] * cr[1] + cu[2] * cr[2]);
-        double mkl = vm * ((1.0 + (0 == r)) * S1[s] - (1.0 + (0 == s)) * S1[r] - (1.0 + (1 == r)) * S0[s] +
-                           (1.0 + (1 == s)) * S0[r]);
-        if (l >= 1 && l <= 4 && ((rc6 >> (53 + l)) & 1)) {
-          ckl = -ckl;
-          mkl = -mkl;
+        // the middle terms in the order of (higher edge, lower edge)
+        const double qr = (q == r ? 2.0 : 1.0) * Sp[u], pu = (p == u ? 2.0 : 1.0) * Sq[r];
+        double mkl = vm * ((p == r ? 2.0 : 1.0) * Sq[u] - (k >= l ? pu : qr) - (k >= l ? qr : pu) +
+                           (q == u ? 2.0 : 1.0) * Sp[r]);
+        if (row_bdr || ((rc6 >> (58 + l)) & 1)) {
+          if (k != l) ckl = 0.0;
+          mkl = 0.0;
         }
-        if (cut) ckl = 0.0;
-        if (cut || row_bdr) mkl = 0.0;
         int pos = (int)((rc6 >> (9 * l)) & kSearch);
-        if (pos == (int)kSearch) {
-          const int i0 = l < 3 ? p : (l < 5 ? q : u), i1 = l == 0 ? q : (l == 1 || l == 3 ? u : w);
-          pos = find_col(ci, kb, ke, __ldg(in.cedge + 6 * (long)t + kEdgeOf(min(i0, i1), max(i0, i1)))) - kb;
-        }
+        if (pos == (int)kSearch) pos = find_col(ci, kb, ke, __ldg(in.cedge + 6 * (long)t + l)) - kb;
         if (tiled) {
           double2 &s2 = tile[kb - s0 + pos];
           s2 = make_double2(s2.x + ckl, s2.y + mkl);

@@ -58,3 +58,37 @@ def test_fan_matches_oracle(n_ring, n_axis, shuffle):
     assert np.abs(C - Co).max() <= 1e-12 * np.abs(Co).max()
     assert np.abs(M - Mo).max() <= 1e-12 * max(np.abs(Mo).max(), 1e-300)
     assert np.array_equal(C, C2) and np.array_equal(M, M2)  # a fixed summation order
+
+
+def _not_mirrored(rp, ci, v):
+    """Entries that differ in any bit from the transposed ones."""
+    n = rp.size - 1
+    row = np.repeat(np.arange(n, dtype=np.int64), np.diff(rp))
+    back = np.lexsort((row, ci))  # entry (j, i) in the place of (i, j): the pattern is symmetric
+    assert np.array_equal(row[back], ci) and np.array_equal(ci[back], row)
+    return int((v != v[back]).sum())
+
+
+@pytest.mark.parametrize("mesh", ["fan-3", "fan-40", "fan-200", "csem_small", "mt_aniso"])
+def test_entries_equal_their_mirror(mesh, request):
+    """C and Ms are symmetric to the bit: both rows of an off-diagonal entry
+    evaluate its one or two terms with the same operands in the same order
+    (the preconditioned iterations assume a symmetric operator, and in the air
+    rounding of C is not small against w Ms)."""
+    if mesh.startswith("fan"):
+        n = int(mesh[4:])
+        m = _fan(n, {3: 2, 40: 3, 200: 6}[n], True)
+        model = mg.Model(mg.ARBITRARY, np.array([[10.0, 30.0, 5.0, 20.0, -35.0, 50.0], [1.0, 2.0, 4.0, 10.0, 0.0, 5.0],
+                                                 [1e8, 1e8, 1e8, 0.0, 0.0, 0.0]]))
+    else:
+        prob = request.getfixturevalue(mesh)
+        m, model = prob.mesh, prob.model
+    with E.EMContext(0) as c:
+        c.set_mesh(m)
+        c.set_model(model)
+        c.set_frequencies([2.0])
+        c.create_linear_system(0)
+        c.assemble_matrix(0)
+        rp, ci = c.make_sparsity_patterns()
+        C, M, _ = c.get_matrices()
+    assert _not_mirrored(rp, ci, C) == 0 and _not_mirrored(rp, ci, M) == 0
