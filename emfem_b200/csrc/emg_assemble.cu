@@ -87,6 +87,11 @@ void build_sparsity(Context &c) {
     std::vector<int> buf;
 #pragma omp for schedule(dynamic, 4096)
     for (int e = 0; e < ne; ++e) {
+      // the order in which a row sums its diagonal: by place within 32 tets, the
+      // order a warp per 32 tets adds them in.  A diagonal that is rounded another
+      // way moves solutions in the air by some 1e-10, so the order is kept.
+      std::sort(e2t.begin() + e2t_rp[e], e2t.begin() + e2t_rp[e + 1],
+                [](int a, int b) { return (a & 31) != (b & 31) ? (a & 31) < (b & 31) : a < b; });
       buf.clear();
       for (int k = e2t_rp[e]; k < e2t_rp[e + 1]; ++k)
         for (int i = 0; i < 6; ++i) buf.push_back(c.h_t2e[6 * (size_t)e2t[k] + i]);

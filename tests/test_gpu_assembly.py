@@ -8,6 +8,8 @@ Bars of the other assembly tests: pattern and boundary cells equal, values to
 1e-12 of the largest.
 """
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -92,3 +94,41 @@ def test_entries_equal_their_mirror(mesh, request):
         rp, ci = c.make_sparsity_patterns()
         C, M, _ = c.get_matrices()
     assert _not_mirrored(rp, ci, C) == 0 and _not_mirrored(rp, ci, M) == 0
+
+
+@pytest.mark.parametrize("mesh", ["fan-40", "fan-200", "csem_small"])
+def test_diagonal_is_summed_in_a_fixed_order(mesh, request):
+    """A diagonal entry is the sum of its tets' entries in the order (t mod 32,
+    t), to the bit: the order of the tet-wise scatter (a warp per 32 tets), which
+    solutions in the air depend on.  The tets' own entries come from a mesh
+    of the same tets with no vertex in common."""
+    if mesh.startswith("fan"):
+        n = int(mesh[4:])
+        m = _fan(n, {40: 3, 200: 6}[n], True)
+        model = mg.Model(mg.ISOTROPIC, np.array([[10.0], [3.0], [1e8]]))
+    else:
+        prob = request.getfixturevalue(mesh)
+        m, model = prob.mesh, prob.model
+    nt = m.n_tets
+    # vertex 4 t + rank keeps the order of a tet's ids, so its entries are the same numbers
+    rank = np.argsort(np.argsort(m.tets, axis=1), axis=1)
+    pts = np.empty((4 * nt, 3))
+    alone = (4 * np.arange(nt)[:, None] + rank).astype(np.int64)
+    pts[alone] = m.points[m.tets]
+    apart = mg.build_topology(pts, alone, m.attr)
+    diag = []
+    for x in (m, apart):
+        x = dataclasses.replace(x, edge_bdr=np.zeros_like(x.edge_bdr))  # no Dirichlet rows: whole entries
+        with E.EMContext(0) as c:
+            c.set_mesh(x)
+            c.set_model(model)
+            c.set_frequencies([2.0])
+            c.create_linear_system(0)
+            c.assemble_matrix(0)
+            rp, ci = c.make_sparsity_patterns()
+            C, _, _ = c.get_matrices()
+        diag.append(C[ci == np.repeat(np.arange(rp.size - 1), np.diff(rp))])
+    want = np.zeros(m.n_edges)
+    for t in np.lexsort((np.arange(nt), np.arange(nt) % 32)):
+        want[m.tet2edge[t]] += diag[1][apart.tet2edge[t]]
+    assert np.array_equal(diag[0], want)
