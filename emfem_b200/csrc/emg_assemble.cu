@@ -65,6 +65,8 @@ void sigma_table(int aniso_form, int nrho, int ncol, const double *rho, std::vec
   }
 }
 
+static void build_incidence(Context &c, const std::vector<int> &e2t_rp);
+
 // ---------------------------------------------------------------------------
 // host: CSR pattern = make_sparsity_patterns (src/em_fwd.cc:191-246)
 // row e: sorted unique edges sharing a tet with e (diagonal included)
@@ -87,11 +89,6 @@ void build_sparsity(Context &c) {
     std::vector<int> buf;
 #pragma omp for schedule(dynamic, 4096)
     for (int e = 0; e < ne; ++e) {
-      // the order in which a row sums its diagonal: by place within 32 tets, the
-      // order a warp per 32 tets adds them in.  A diagonal that is rounded another
-      // way moves solutions in the air by some 1e-10, so the order is kept.
-      std::sort(e2t.begin() + e2t_rp[e], e2t.begin() + e2t_rp[e + 1],
-                [](int a, int b) { return (a & 31) != (b & 31) ? (a & 31) < (b & 31) : a < b; });
       buf.clear();
       for (int k = e2t_rp[e]; k < e2t_rp[e + 1]; ++k)
         for (int i = 0; i < 6; ++i) buf.push_back(c.h_t2e[6 * (size_t)e2t[k] + i]);
@@ -119,9 +116,7 @@ void build_sparsity(Context &c) {
   c.rp.upload(c.h_rp, c.stream);
   c.ci.upload(c.h_ci, c.stream);
   c.chunk_rp.release();
-  c.einc_rp.upload(e2t_rp, c.stream);
-  c.einc.upload(e2t, c.stream);
-  EMG_CUDA(cudaStreamSynchronize(c.stream));  // the incidence lists go out of scope
+  build_incidence(c, e2t_rp);
 }
 
 // vertex adjacency (pattern of G^T B G and Pi^T B Pi) and vertex->edge incidence
@@ -176,6 +171,73 @@ __device__ __forceinline__ int find_col(const int *__restrict__ ci, int b, int e
   return lo;
 }
 
+// Tets around each edge (in any order) and the interior faces 4 t + f of their
+// lower tet, for estimate_face_kernel: a block's faces lie together
+__global__ void __launch_bounds__(256) incidence_kernel(int nt, const int *__restrict__ t2e,
+                                                        const int *__restrict__ nbr, const int *__restrict__ inc_rp,
+                                                        int *__restrict__ cursor, int *__restrict__ inc,
+                                                        int *__restrict__ n_faces, int *__restrict__ faces) {
+  __shared__ int warp_sum[8], base;
+  const int t = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned mine = 0;  // bit f: face f is listed here
+  if (t < nt) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int e = __ldg(t2e + 6 * (long)t + k);
+      inc[__ldg(inc_rp + e) + atomicAdd(cursor + e, 1)] = t;
+    }
+    const int4 nb = __ldg(reinterpret_cast<const int4 *>(nbr) + t);
+    mine = (nb.x > t ? 1u : 0u) | (nb.y > t ? 2u : 0u) | (nb.z > t ? 4u : 0u) | (nb.w > t ? 8u : 0u);
+  }
+  const int n = __popc(mine);
+  int upto = n;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, off);
+    if (lane >= off) upto += v;
+  }
+  if (lane == 31) warp_sum[warp] = upto;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < 8; ++w) {
+      const int v = warp_sum[w];
+      warp_sum[w] = sum;
+      sum += v;
+    }
+    base = atomicAdd(n_faces, sum);
+  }
+  __syncthreads();
+  int o = base + warp_sum[warp] + upto - n;
+  for (int f = 0; f < 4; ++f)
+    if ((mine >> f) & 1) faces[o++] = 4 * t + f;
+}
+
+// Device copies of the incidence (its row pointer comes from the pattern's
+// host pass) and the face list.  One allocation holds them with the assembly
+// records: below a megabyte cudaMalloc takes 350 us where it needs a new
+// driver slab, above it always.
+static void build_incidence(Context &c, const std::vector<int> &e2t_rp) {
+  c.n_faces = 0;
+  for (long i = 0; i < 4L * c.nt; ++i) c.n_faces += c.h_nbr[i] > i / 4;
+  const size_t n6 = 6 * (size_t)c.nt;
+  const size_t recs = std::max(n6, ((size_t)c.ne + 1) / 2);  // the cursors lie there first
+  const size_t ints = n6 + (size_t)c.ne + 1 + (size_t)c.n_faces + 1;
+  c.inc_mem.alloc(recs + (ints + 1) / 2);
+  c.erec = c.inc_mem.p;
+  c.einc = reinterpret_cast<int *>(c.erec + recs);
+  c.einc_rp = c.einc + n6;
+  c.faces = c.einc_rp + c.ne + 1;
+  int *count = c.faces + c.n_faces, *cursor = reinterpret_cast<int *>(c.erec);
+  EMG_CUDA(cudaMemcpyAsync(c.einc_rp, e2t_rp.data(), sizeof(int) * ((size_t)c.ne + 1), cudaMemcpyHostToDevice,
+                           c.stream));
+  EMG_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)c.ne, c.stream));
+  EMG_CUDA(cudaMemsetAsync(count, 0, sizeof(int), c.stream));
+  incidence_kernel<<<(unsigned)((c.nt + 255) / 256), 256, 0, c.stream>>>(c.nt, c.t2e.p, c.nbr.p, c.einc_rp, cursor,
+                                                                         c.einc, count, c.faces);
+  EMG_LAUNCH_CHECK();
+}
+
 // Record of an (edge, tet) incidence for assemble_edge_kernel:
 //   einc[j]: the tet, with the edge's canonical index k in bits 28..30
 //   erec[j]: per canonical edge l of the tet 9 bits, its position in the
@@ -184,6 +246,35 @@ __device__ __forceinline__ int find_col(const int *__restrict__ ci, int b, int e
 constexpr int kTetBits = 28;
 constexpr unsigned kSearch = 511;
 
+// The tets of an edge in the order in which its row sums the diagonal: by place
+// within 32 tets, the order a warp per 32 tets adds them in.  A diagonal that is
+// rounded another way moves solutions in the air by some 1e-10, so the order
+// is kept.
+__device__ __forceinline__ unsigned sum_order(int t) { return ((unsigned)(t & 31) << (kTetBits - 5)) | (unsigned)(t >> 5); }
+
+// heap sort of one edge's list (5 tets as a rule, hundreds in a fan)
+__device__ void sort_tets(int *a, int n) {
+  auto sift = [&](int root, int end) {
+    const int v = a[root];
+    for (;;) {
+      int child = 2 * root + 1;
+      if (child >= end) break;
+      if (child + 1 < end && sum_order(a[child + 1]) > sum_order(a[child])) ++child;
+      if (sum_order(a[child]) <= sum_order(v)) break;
+      a[root] = a[child];
+      root = child;
+    }
+    a[root] = v;
+  };
+  for (int i = n / 2 - 1; i >= 0; --i) sift(i, n);
+  for (int end = n - 1; end > 0; --end) {
+    const int v = a[0];
+    a[0] = a[end];
+    a[end] = v;
+    sift(0, end);
+  }
+}
+
 __global__ void edge_records_kernel(int ne, const int *__restrict__ inc_rp, int *__restrict__ inc,
                                     const int *__restrict__ cedge, const unsigned char *__restrict__ ebdr,
                                     const int *__restrict__ rp, const int *__restrict__ ci,
@@ -191,7 +282,9 @@ __global__ void edge_records_kernel(int ne, const int *__restrict__ inc_rp, int 
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const int kb = __ldg(rp + e), ke = __ldg(rp + e + 1);
-  for (int j = __ldg(inc_rp + e); j < __ldg(inc_rp + e + 1); ++j) {
+  const int j0 = __ldg(inc_rp + e), j1 = __ldg(inc_rp + e + 1);
+  sort_tets(inc + j0, j1 - j0);
+  for (int j = j0; j < j1; ++j) {
     const int t = inc[j];
     unsigned long long r = 0;
     int k = 0;
@@ -230,9 +323,8 @@ __global__ void vslot_map_kernel(int nt, const int *__restrict__ tets, const int
 
 void build_slot_maps(Context &c) {
   if (c.nt >= (1 << kTetBits)) fail(EMG_ERR_ARG, "mesh of %d tets", c.nt);
-  c.erec.alloc((size_t)c.nt * 6);
-  edge_records_kernel<<<(unsigned)((c.ne + 127) / 128), 128, 0, c.stream>>>(c.ne, c.einc_rp.p, c.einc.p, c.cedge.p,
-                                                                            c.ebdr.p, c.rp.p, c.ci.p, c.erec.p);
+  edge_records_kernel<<<(unsigned)((c.ne + 127) / 128), 128, 0, c.stream>>>(c.ne, c.einc_rp, c.einc, c.cedge.p,
+                                                                            c.ebdr.p, c.rp.p, c.ci.p, c.erec);
   EMG_LAUNCH_CHECK();
   c.bdr_cell.alloc(c.nt);
   bdr_cell_kernel<<<(unsigned)((c.nt + 255) / 256), 256, 0, c.stream>>>(c.nt, c.cedge.p, c.ebdr.p, c.bdr_cell.p);
@@ -478,7 +570,7 @@ void assemble_edge(Context &c) {
   c.Cv.alloc(c.nnz);
   c.Msv.alloc(c.nnz);
   assemble_edge_kernel<<<(unsigned)((c.ne + ASM_ROWS - 1) / ASM_ROWS), ASM_ROWS, 0, c.stream>>>(
-      elem_in(c), c.ne, c.einc_rp.p, c.einc.p, c.erec.p, c.rp.p, c.ci.p, c.Cv.p, c.Msv.p);
+      elem_in(c), c.ne, c.einc_rp, c.einc, c.erec, c.rp.p, c.ci.p, c.Cv.p, c.Msv.p);
   EMG_LAUNCH_CHECK();
 }
 

@@ -843,7 +843,6 @@ int emg_set_mesh(emg_context *c, int nv, const double *pts, int nt, const int *t
   c->non.upload(c->h_non, c->stream);
   c->ebdr.upload(c->h_ebdr, c->stream);
   canonicalize(*c);
-  build_faces(*c);
   EMG_CUDA(cudaStreamSynchronize(c->stream));
   EMG_API_END
 }
@@ -917,9 +916,7 @@ int emg_destroy_linear_system(emg_context *c) {
   need(c != nullptr, EMG_ERR_ARG, "null context");
   c->Cv.release();
   c->Msv.release();
-  c->einc.release();
-  c->einc_rp.release();
-  c->erec.release();
+  c->inc_mem.release();
   c->vslot.release();
   c->rp.release();
   c->ci.release();

@@ -283,18 +283,6 @@ __global__ void __launch_bounds__(128) estimate_cell_kernel(EstIn in, int nt, co
     if (s < in.nsol - 1) err[(long)s * nt + t] = sqrt(es[s] * dual);
 }
 
-// interior faces from the lower tet's side, for estimate_face_kernel
-void build_faces(Context &c) {
-  std::vector<int> f;
-  f.reserve(2 * (size_t)c.nt);
-  for (int t = 0; t < c.nt; ++t)
-    for (int k = 0; k < 4; ++k)
-      if (c.h_nbr[4 * (size_t)t + k] > t) f.push_back(4 * t + k);
-  c.n_faces = (int)f.size();
-  c.faces.upload(f, c.stream);
-  EMG_CUDA(cudaStreamSynchronize(c.stream));
-}
-
 void launch_estimate(Context &c, double omega, int nsol, const double *const *sol_dev, double *eta_dev,
                      double *err_dev, double *scratch_fe) {
   EstIn in;
@@ -311,7 +299,7 @@ void launch_estimate(Context &c, double omega, int nsol, const double *const *so
   for (int s = 0; s < 3; ++s) in.sol[s] = s < nsol ? (const double2 *)sol_dev[s] : nullptr;
   in.omega = omega;
   if (c.n_faces > 0) {
-    estimate_face_kernel<<<(unsigned)((c.n_faces + 127) / 128), 128, 0, c.stream>>>(in, c.nt, c.n_faces, c.faces.p,
+    estimate_face_kernel<<<(unsigned)((c.n_faces + 127) / 128), 128, 0, c.stream>>>(in, c.nt, c.n_faces, c.faces,
                                                                                     scratch_fe);
     EMG_LAUNCH_CHECK();
   }

@@ -316,8 +316,6 @@ struct Context {
   DBuf<unsigned char> ebdr;
   DBuf<int> ctet, cedge;           // canonical tets: sorted vertices, canonical edges
   DBuf<signed char> cpar;          // parity of the vertex sort
-  DBuf<int> faces;                 // interior faces, 4 t + f of their lower tet
-  int n_faces = 0;
   // model
   int aniso_form = 0;
   std::vector<double> rho;
@@ -337,8 +335,10 @@ struct Context {
   DBuf<int> rp, ci;
   DBuf<int> chunk_rp;              // chunk row pointer of the pattern (SpmmArgs::crp), built on first use
   long n_chunks = 0;
-  DBuf<int> einc_rp, einc;         // tets around each edge (6 per tet in all)
-  DBuf<unsigned long long> erec;   // their records for the assembly (edge_records_kernel)
+  DBuf<unsigned long long> inc_mem;     // holds the next four
+  unsigned long long *erec = nullptr;   // records of the incidences for the assembly (edge_records_kernel)
+  int *einc = nullptr, *einc_rp = nullptr;  // tets around each edge (6 per tet in all)
+  int *faces = nullptr, n_faces = 0;    // interior faces, 4 t + f of their lower tet (estimator)
   DBuf<double> Cv, Msv;            // C and Ms (omega-free mass) on the pattern
   DBuf<unsigned char> bdr_cell;
   bool assembled = false;
@@ -390,10 +390,9 @@ void set_last_error(const char *msg);
 
 // helpers implemented in the .cu/.cpp files
 void sigma_table(int aniso_form, int nrho, int ncol, const double *rho, std::vector<double> &out);
-void build_sparsity(Context &c);          // host: CSR pattern (make_sparsity_patterns)
+void build_sparsity(Context &c);          // host: CSR pattern (make_sparsity_patterns); device: incidence, faces
 void build_vertex_pattern(Context &c);    // host: vertex adjacency + incidence
 void canonicalize(Context &c);            // device: sorted tets + canonical edges
-void build_faces(Context &c);             // the interior face list (estimator)
 void build_slot_maps(Context &c);         // device: edge incidence records, tet -> vertex CSR slots
 void assemble_edge(Context &c);           // device: C, Ms, bdr cells
 void assemble_nodal(Context &c, HCsr out[4]);  // device + download (G, Pi_x, Pi_y, Pi_z)
