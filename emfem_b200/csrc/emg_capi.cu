@@ -93,65 +93,82 @@ void DevicePool::trim() {
   cached = 0;
 }
 
-PinnedStage::PinnedStage() {
-  for (int i = 0; i < 2; ++i) {
-    const cudaError_t e = cudaHostAlloc((void **)&buf[i], kBytes, cudaHostAllocPortable);
-    if (e == cudaSuccess) continue;
-    buf[i] = nullptr;
-    if (i) cudaFreeHost(buf[0]);
-    EMG_CUDA(e);
-  }
-}
+namespace {
 
-PinnedStage::~PinnedStage() {
-  for (int i = 0; i < 2; ++i)
-    if (buf[i]) cudaFreeHost(buf[i]);
-}
+struct PinnedStage {
+  static constexpr size_t kBytes = size_t(1) << 20;  // each buffer; both fill one pinned slab of the driver
+  char *buf[2] = {nullptr, nullptr};
+  std::mutex mu;  // one copy at a time
+};
 
-std::shared_ptr<PinnedStage> PinnedStage::get() {
+// the process's buffers, kept until it exits; null for its first result, or
+// where they cannot be had
+PinnedStage *pinned_stage() {
   static std::mutex mu;
-  static std::weak_ptr<PinnedStage> shared;
+  static PinnedStage *stage = nullptr;
+  static bool asked = false, refused = false;
   std::lock_guard<std::mutex> lock(mu);
-  std::shared_ptr<PinnedStage> p = shared.lock();
-  if (!p) shared = p = std::make_shared<PinnedStage>();
-  return p;
+  if (stage || refused) return stage;
+  if (!asked) {
+    asked = true;
+    return nullptr;
+  }
+  char *p = nullptr;
+  if (cudaHostAlloc((void **)&p, 2 * PinnedStage::kBytes, cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    refused = true;
+    return nullptr;
+  }
+  stage = new PinnedStage;
+  stage->buf[0] = p;
+  stage->buf[1] = p + PinnedStage::kBytes;
+  return stage;
 }
+
+}  // namespace
 
 StagedCopy::~StagedCopy() {
   for (int i = 0; i < 2; ++i)
     if (done[i]) cudaEventDestroy(done[i]);
 }
 
-void StagedCopy::open() {
-  if (!stage) stage = PinnedStage::get();
-  for (int i = 0; i < 2; ++i)
-    if (!done[i]) EMG_CUDA(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
-}
-
 void StagedCopy::download(void *host, const void *dev, size_t bytes, cudaStream_t s) {
   if (bytes == 0) return;
-  open();
-  std::lock_guard<std::mutex> lock(stage->mu);
-  constexpr size_t kBytes = PinnedStage::kBytes;
+  constexpr size_t kBytes = PinnedStage::kBytes, kSmall = size_t(16) << 10, kOmpBytes = size_t(1) << 20;
+  PinnedStage *stage = bytes > kSmall ? pinned_stage() : nullptr;
+  std::unique_lock<std::mutex> lock;
+  if (stage) lock = std::unique_lock<std::mutex>(stage->mu, std::try_to_lock);
+  if (!lock.owns_lock()) {
+    EMG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, s));
+    EMG_CUDA(cudaStreamSynchronize(s));
+    return;
+  }
   char *const *buf = stage->buf;
   const long n = (long)((bytes + kBytes - 1) / kBytes);
   auto size = [&](long i) { return std::min(kBytes, bytes - (size_t)i * kBytes); };
-  for (long i = 0; i <= n; ++i) {
-    if (i < n) {
-      EMG_CUDA(cudaMemcpyAsync(buf[i & 1], (const char *)dev + (size_t)i * kBytes, size(i), cudaMemcpyDeviceToHost, s));
-      EMG_CUDA(cudaEventRecord(done[i & 1], s));
-    }
-    if (i == 0) continue;
-    EMG_CUDA(cudaEventSynchronize(done[(i - 1) & 1]));
-    char *to = (char *)host + (size_t)(i - 1) * kBytes;
-    const char *from = buf[(i - 1) & 1];
-    const long m = (long)size(i - 1);
-    constexpr long kPart = 64 << 10;
-    constexpr size_t kOmpBytes = 1 << 20;
-    const long parts = (m + kPart - 1) / kPart;
-    // waking the host threads pays from about a megabyte on
+  try {
+    for (int i = 0; i < 2; ++i)
+      if (!done[i]) EMG_CUDA(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
+    for (long i = 0; i <= n; ++i) {
+      if (i < n) {
+        EMG_CUDA(cudaMemcpyAsync(buf[i & 1], (const char *)dev + (size_t)i * kBytes, size(i), cudaMemcpyDeviceToHost,
+                                 s));
+        EMG_CUDA(cudaEventRecord(done[i & 1], s));
+      }
+      if (i == 0) continue;
+      EMG_CUDA(cudaEventSynchronize(done[(i - 1) & 1]));
+      char *to = (char *)host + (size_t)(i - 1) * kBytes;
+      const char *from = buf[(i - 1) & 1];
+      const long m = (long)size(i - 1);
+      constexpr long kPart = 64 << 10;
+      const long parts = (m + kPart - 1) / kPart;
+      // waking the host threads pays from about a megabyte on
 #pragma omp parallel for schedule(static) if (bytes > kOmpBytes)
-    for (long q = 0; q < parts; ++q) std::memcpy(to + q * kPart, from + q * kPart, std::min(kPart, m - q * kPart));
+      for (long q = 0; q < parts; ++q) std::memcpy(to + q * kPart, from + q * kPart, std::min(kPart, m - q * kPart));
+    }
+  } catch (...) {
+    cudaStreamSynchronize(s);  // a copy in flight must not reach the buffers of the next result
+    throw;
   }
 }
 
@@ -712,7 +729,6 @@ int emg_create_context(emg_context **ctx, int device) {
     // the allocation-free estimator's scratch address, looked up now so that
     // its module is loaded and the address cached before any run
     (void)noalloc_scratch_address(device);
-    c->stage.open();
   } catch (...) {
     delete c;
     throw;

@@ -166,29 +166,16 @@ struct DBuf {
 // Copies device results to pageable host memory through two pinned buffers: the
 // GPU fills one while the host's threads empty the other.  The driver's own
 // copy to pageable memory goes through one thread (12 MB of error indicators:
-// 1.5 ms).  One pair of buffers serves every device context of the process,
-// one copy at a time (pinning them takes milliseconds); the last context gives
-// them back.
-struct PinnedStage {
-  static constexpr size_t kBytes = size_t(2) << 20;  // each buffer
-  char *buf[2] = {nullptr, nullptr};
-  std::mutex mu;
-  PinnedStage();
-  PinnedStage(const PinnedStage &) = delete;
-  PinnedStage &operator=(const PinnedStage &) = delete;
-  ~PinnedStage();
-  static std::shared_ptr<PinnedStage> get();
-};
-
-// a context's way through it
+// 1.5 ms).  One pair of buffers, 2 MB in all, serves the process: pinning them
+// takes 1.3 to 2.8 ms, so the first result of the process goes the driver's way
+// and they are kept from the second on.  So does a result that finds
+// them in use, and one too small to gain: a call never waits for another context.
 struct StagedCopy {
-  std::shared_ptr<PinnedStage> stage;
   cudaEvent_t done[2] = {nullptr, nullptr};
   StagedCopy() = default;
   StagedCopy(const StagedCopy &) = delete;
   StagedCopy &operator=(const StagedCopy &) = delete;
   ~StagedCopy();
-  void open();  // buffers and events; the context's device is current
   // returns when host[0 .. bytes) is written
   void download(void *host, const void *dev, size_t bytes, cudaStream_t s);
 };
