@@ -48,51 +48,6 @@ void launch_check(const char *file, int line) {
   check_cuda(cudaGetLastError(), "kernel launch", file, line);
 }
 
-DevicePool *&current_pool() {
-  static thread_local DevicePool *p = nullptr;
-  return p;
-}
-
-void *DevicePool::get(size_t &bytes) {
-  bytes = (bytes + 511) / 512 * 512;
-  // a block up to an eighth (and 64 KB) larger than asked for
-  auto it = blocks.lower_bound(bytes);
-  if (it != blocks.end() && it->first <= bytes + bytes / 8 + 65536) {
-    void *p = it->second;
-    bytes = it->first;
-    cached -= bytes;
-    blocks.erase(it);
-    return p;
-  }
-  void *p = nullptr;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
-    (void)cudaGetLastError();
-    if (blocks.empty()) break;
-    trim();
-  }
-  return nullptr;
-}
-
-void DevicePool::put(void *p, size_t bytes) {
-  if (cached + bytes > kPoolKeep) {
-    cudaFree(p);
-    return;
-  }
-  try {
-    blocks.emplace(bytes, p);
-    cached += bytes;
-  } catch (...) {
-    cudaFree(p);
-  }
-}
-
-void DevicePool::trim() {
-  for (auto &b : blocks) cudaFree(b.second);  // waits for the GPU
-  blocks.clear();
-  cached = 0;
-}
-
 namespace {
 
 struct PinnedStage {
@@ -725,6 +680,7 @@ int emg_create_context(emg_context **ctx, int device) {
     delete c;
     check_cuda(e, "cudaStreamCreate", __FILE__, __LINE__);
   }
+  c->pool.join(DevicePool::of(device), c->stream);
   try {
     // the allocation-free estimator's scratch address, looked up now so that
     // its module is loaded and the address cached before any run
@@ -848,7 +804,7 @@ int emg_set_mesh(emg_context *c, int nv, const double *pts, int nt, const int *t
   c->have_pc = false;
   c->ws->block_ready64 = c->ws->block_ready32 = false;
   c->sol.clear();
-  c->pool.trim();
+  if (c->device >= 0) c->pool.pool->trim(&c->pool);
   if (c->device < 0) return EMG_OK;  // host-only context: host-side entry points only
   c->pts.upload(c->h_pts, c->stream);
   c->tets.upload(c->h_tets, c->stream);
@@ -940,7 +896,7 @@ int emg_destroy_linear_system(emg_context *c) {
   c->have_ls = c->assembled = c->have_pc = false;
   c->ws->block_ready64 = c->ws->block_ready32 = false;
   if (c->device >= 0) EMG_CUDA(cudaSetDevice(c->device));
-  c->pool.trim();
+  if (c->device >= 0) c->pool.pool->trim(&c->pool);
   EMG_API_END
 }
 

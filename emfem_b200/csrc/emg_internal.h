@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/emfem_b200.h"
+#include "emg_pool.h"
 
 namespace emg {
 
@@ -60,47 +61,14 @@ long launch_count();
 void add_launches(long n);
 
 // ---------------------------------------------------------------------------
-// device memory of a context
-// ---------------------------------------------------------------------------
-// Freed blocks are kept for the context's next allocations: cudaMalloc and
-// cudaFree take 0.1 ms each and now and then tens of milliseconds, an AMS
-// setup needs some 150 of them and a receiver call 4.  A block goes straight
-// back to work without waiting for the GPU, because a context's work runs on
-// its one stream.  At most kPoolKeep bytes stay cached; trim() (called when a
-// linear system or its context is destroyed, a mesh is set, or an allocation
-// fails) gives them back.  Used by one thread at a time, like its context.
-struct DevicePool {
-  static constexpr size_t kPoolKeep = size_t(4) << 30;
-  std::multimap<size_t, void *> blocks;  // by size
-  size_t cached = 0;
-  DevicePool() = default;
-  DevicePool(const DevicePool &) = delete;
-  DevicePool &operator=(const DevicePool &) = delete;
-  ~DevicePool() { trim(); }
-  void *get(size_t &bytes);  // at least `bytes` (set to the block's size); null when out of memory
-  void put(void *p, size_t bytes);
-  void trim();
-};
-
-// the pool that allocations of this thread come from (null: cudaMalloc)
-DevicePool *&current_pool();
-struct PoolScope {
-  DevicePool *before;
-  explicit PoolScope(DevicePool &pool) : before(current_pool()) { current_pool() = &pool; }
-  PoolScope(const PoolScope &) = delete;
-  PoolScope &operator=(const PoolScope &) = delete;
-  ~PoolScope() { current_pool() = before; }
-};
-
-// ---------------------------------------------------------------------------
-// device buffer (from the current pool or cudaMalloc, move-only)
+// device buffer (from the current context's pool or cudaMalloc, move-only)
 // ---------------------------------------------------------------------------
 template <typename T>
 struct DBuf {
   T *p = nullptr;
   size_t n = 0;
-  DevicePool *pool = nullptr;  // where the block came from
-  size_t block = 0;            // its size
+  PoolUser *user = nullptr;  // whose pool the block came from
+  size_t block = 0;          // its size
   DBuf() = default;
   explicit DBuf(size_t count) { alloc(count); }
   DBuf(const DBuf &) = delete;
@@ -117,7 +85,7 @@ struct DBuf {
   void take(DBuf &o) noexcept {
     p = o.p;
     n = o.n;
-    pool = o.pool;
+    user = o.user;
     block = o.block;
     o.p = nullptr;
     o.n = 0;
@@ -126,10 +94,10 @@ struct DBuf {
     if (count == n && p) return;
     release();
     if (count == 0) return;
-    pool = current_pool();
+    user = current_user();
     block = count * sizeof(T);
-    if (pool) {
-      p = static_cast<T *>(pool->get(block));
+    if (user) {
+      p = static_cast<T *>(user->pool->get(block, user));
     } else if (cudaMalloc((void **)&p, block) != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
@@ -138,7 +106,7 @@ struct DBuf {
     n = count;
   }
   void release() {
-    if (p && pool) pool->put(p, block);
+    if (p && user) user->pool->put(p, block, user);
     else if (p) cudaFree(p);
     p = nullptr;
     n = 0;
@@ -288,7 +256,7 @@ struct Workspace;
 // context (mirrors EMContext, em_ctx.h:15-64)
 // ---------------------------------------------------------------------------
 struct Context {
-  DevicePool pool;  // first member: outlives every buffer below
+  PoolUser pool;  // first member: outlives every buffer below
   StagedCopy stage;
   int device = 0;
   cudaStream_t stream = nullptr;

@@ -63,7 +63,15 @@ const char *emg_version(void);
  * or -1 for a host-only context: it takes options, mesh, model, frequencies
  * and background, and serves the host-side entry points (CSEM and dual
  * right-hand sides, point location, marking, responses); every entry point
- * that needs a GPU returns EMG_ERR_STATE. */
+ * that needs a GPU returns EMG_ERR_STATE.
+ * Device memory that contexts free is kept for their next allocations, one
+ * store per device and process: at most 4 GB, and an eighth of the free memory
+ * with it once more than 256 MB are kept.  A context's part goes back to the
+ * driver in emg_set_mesh, emg_destroy_linear_system and emg_destroy_context,
+ * all of it when an allocation of the library fails.  Other allocators of the
+ * process (PyTorch, NCCL) cannot reach it: call one of these before they need
+ * it.  2 MB of pinned host memory are kept from the process's second large
+ * result until it exits. */
 int emg_create_context(emg_context **ctx, int device);
 int emg_destroy_context(emg_context *ctx);
 
