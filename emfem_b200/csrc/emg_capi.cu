@@ -785,6 +785,7 @@ int emg_set_mesh(emg_context *c, int nv, const double *pts, int nt, const int *t
     need(nbr[i] >= -1 && nbr[i] < nt, EMG_ERR_ARG, "neighborlist index out of range");
     need(nbr[i] < 0 || (non[i] >= 0 && non[i] < 4), EMG_ERR_ARG, "tet_non index out of range");
   }
+  ++c->model_version;
   c->nv = nv;
   c->nt = nt;
   c->ne = ne;
@@ -828,6 +829,7 @@ int emg_set_model(emg_context *c, int aniso_form, int n_rho, int ncol, const dou
   if (c->nt) {
     for (int a : c->h_attr) need(a >= 0 && a < n_rho, EMG_ERR_ARG, "tet attribute beyond the resistivity table");
   }
+  ++c->model_version;
   c->aniso_form = aniso_form;
   c->nrho = n_rho;
   c->ncol = ncol;

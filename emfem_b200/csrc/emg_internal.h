@@ -326,6 +326,7 @@ struct Context {
   std::unique_ptr<Workspace> ws;
   // learned warm start (network, optimiser state, per-edge features), built on first use
   std::shared_ptr<struct WarmStartNet> warm;
+  long model_version = 0;          // counts emg_set_mesh and emg_set_model (the features are of one of each)
   Context();
   ~Context();
 };

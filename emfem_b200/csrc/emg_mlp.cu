@@ -687,7 +687,7 @@ void WarmStartNet::statics(Context &c) {
   edge_static_kernel<<<(c.ne + 255) / 256, 256, 0, s>>>(c.ne, c.edges.p, c.pts.p, acc.p, stat.p);
   EMG_LAUNCH_CHECK();
   EMG_CUDA(cudaStreamSynchronize(s));  // temporaries go out of scope
-  stat_ne = c.ne;
+  stat_version = c.model_version;
 }
 
 static void launch_mlp(int mode, const KArgs &a, int grid, cudaStream_t s) {

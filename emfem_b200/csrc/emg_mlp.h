@@ -39,7 +39,7 @@ struct WarmStartNet {
   double last_loss = -1, last_loss0 = -1;
   DBuf<int> err;
   DBuf<float4> stat;             // 3 per edge
-  int stat_ne = 0;
+  long stat_version = -1;        // Context::model_version they belong to
   DBuf<Spec> specs_dev;
   void init(uint64_t seed, cudaStream_t s);
   void set_params(const float *host, cudaStream_t s);

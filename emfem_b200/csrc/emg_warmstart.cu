@@ -139,7 +139,7 @@ PoolScope prepare(Context &c, WarmStartNet &net, unsigned seed) {
   {
     const PoolScope on(c.pool);
     if (!net.ready) net.init(seed, c.stream);
-    if (net.stat_ne != c.ne || !net.stat.p) net.statics(c);
+    if (net.stat_version != c.model_version) net.statics(c);
   }
   return PoolScope(c.pool);
 }

@@ -202,3 +202,49 @@ def test_warm_start_ab_iterations(ab_runs):
     for arm in ("interp", "network", "auto"):
         assert np.all(ab_runs[arm]["r0"] <= 1.0)
     assert sum(ab_runs["auto"]["its"]) <= sum(ab_runs["zero"]["its"])
+
+
+@pytest.mark.parametrize("change", ["model", "mesh"])
+def test_prediction_follows_model_and_mesh(small, change):
+    """The network's per-edge features are those of the current model and mesh:
+    after a new one of the same size a context predicts what a fresh context
+    with the same parameters does (the module's 2e-3), not what it did before."""
+    import dataclasses
+    import torch
+    prob, xd = small["prob"], small["xd"]
+    par = _random_params(np.random.default_rng(21))
+    rho = prob.model.rho.copy()
+    rho[1:] *= 30.0
+    new_model = mg.Model(prob.model.aniso_form, rho if change == "model" else prob.model.rho)
+    new_mesh = prob.mesh if change == "model" else dataclasses.replace(prob.mesh, points=prob.mesh.points * [1, 1, 2.5])
+    tf, ts = np.array([0.3, 3.0, 0.3, 3.0]), np.array([0, 0, 1, 1], dtype=np.int32)
+
+    def correction(c):
+        out = []
+        for net in (1, 0):
+            g = torch.empty((prob.mesh.n_edges, 4), dtype=torch.complex128, device="cuda")
+            c.warm_start_predict(small["freqs"], small["src"], xd.data_ptr(), tf, ts, g.data_ptr(), network=net)
+            out.append(g.cpu().numpy())
+        return out[0] - out[1]
+
+    def setup(c, mesh, model):
+        c.set_mesh(mesh)
+        c.set_model(model)
+        c.set_frequencies(prob.survey.freqs)
+        c.create_linear_system(-3)
+
+    with E.EMContext(0) as c, E.EMContext(0) as fresh:
+        setup(c, prob.mesh, prob.model)
+        c.warm_start_params(set_to=par)
+        before = correction(c)
+        if change == "model":
+            c.set_model(new_model)
+        else:
+            setup(c, new_mesh, new_model)
+        after = correction(c)
+        setup(fresh, new_mesh, new_model)
+        fresh.warm_start_params(set_to=par)
+        want = correction(fresh)
+    big = np.abs(want).max(axis=0)
+    assert (np.abs(want - before).max(axis=0) > 0.02 * big).all()  # the features matter
+    assert (np.abs(want - after).max(axis=0) <= 2e-3 * big).all()
