@@ -184,8 +184,8 @@ def orient3d_sign(a, b, c, d) -> int:
 
 def spmm_layouts() -> str:
     """The SpMM lane layouts the autotuner chose so far (text)."""
-    buf = C.create_string_buffer(4096)
-    _check(lib().emg_spmm_layouts(buf, 4096))
+    buf = C.create_string_buffer(1 << 16)
+    _check(lib().emg_spmm_layouts(buf, len(buf)))
     return buf.value.decode()
 
 

@@ -177,7 +177,21 @@ SpmmTuner &tuner() {
   return t;
 }
 
-std::string SpmmTuner::report() const {
+bool SpmmTuner::find(const Key &k, Layout &l) {
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = best.find(k);
+  if (it == best.end()) return false;
+  l = it->second;
+  return true;
+}
+
+SpmmTuner::Layout SpmmTuner::add(const Key &k, const Layout &l) {
+  std::lock_guard<std::mutex> lock(mu);
+  return best.emplace(k, l).first->second;
+}
+
+std::string SpmmTuner::report() {
+  std::lock_guard<std::mutex> lock(mu);
   std::ostringstream os;
   for (auto &kv : best)
     os << "T" << std::get<0>(kv.first) * 8 << " K" << std::get<1>(kv.first) << " nnz/row class "
@@ -239,18 +253,14 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
   const bool packed = a.pk != nullptr && sizeof(T) == 4 && a.vm != nullptr;
   const bool chunked = a.ch != nullptr && a.crp != nullptr && sizeof(T) == 4 && a.vm != nullptr;
   auto key = std::make_tuple((int)sizeof(T), K, bucket, 4 * size_class(a) + (packed ? 1 : 0) + (chunked ? 2 : 0));
-  auto it = tn.best.find(key);
-  std::pair<int, int> cfg;
-  if (it != tn.best.end() && (long)a.n * (K / spmm_default<T>(K, 1.0).first) >= kLaneSlots) {
-    cfg = it->second;
-  } else {
-    cfg = spmm_default<T>(K, a.n ? (double)nnz / a.n : 1.0);
-    const bool fills = (long)a.n * (K / cfg.first) >= kLaneSlots;
+  SpmmTuner::Layout cfg = spmm_default<T>(K, (double)nnz / a.n);
+  const bool fills = (long)a.n * (K / cfg.first) >= kLaneSlots;
+  if (fills && !tn.find(key, cfg)) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     EMG_CUDA(cudaStreamIsCapturing(s, &cs));
     const bool idempotent = a.mode == SPMM_AX || a.mode == SPMM_RES || a.mode == SPMM_JAC || a.mode == SPMM_CHEB1 ||
                             a.mode == SPMM_AXJ0 || a.mode == SPMM_RESJ0;
-    if (tn.allow_tuning && cs == cudaStreamCaptureStatusNone && idempotent && fills) {
+    if (cs == cudaStreamCaptureStatusNone && idempotent) {
       cudaEvent_t e0, e1;
       EMG_CUDA(cudaEventCreate(&e0));
       EMG_CUDA(cudaEventCreate(&e1));
@@ -258,7 +268,7 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
       // software-pipelined kernel (nl 200 + U / 300 + U) is left out: it won
       // the tuning call's mode by a hair on the MT topography edge matrix and
       // then ran 17% slower over the solver's mix of smoothing modes.
-      std::vector<std::pair<int, int>> cand;
+      std::vector<SpmmTuner::Layout> cand;
       for (int v : {1, 2, 4})
         for (int nl : {1, 2, 4, 8, 16, 32, -4, -8, 101, 102, 104, 401, 402, 501, 502, 601, 604, 801, 802}) {
           if (((nl > 100 && nl < 200) || (nl > 400 && nl < 500)) && !packed) continue;
@@ -290,8 +300,7 @@ void spmm_nnz(int K, const SpmmArgs &a, long nnz, cudaStream_t s) {
         }
       EMG_CUDA(cudaEventDestroy(e0));
       EMG_CUDA(cudaEventDestroy(e1));
-      tn.best[key] = cfg;
-      tn.tuned_count++;
+      cfg = tn.add(key, cfg);
     }
   }
   SpmmFn f = spmm_fn<T>(K, cfg.first, cfg.second);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 
@@ -16,12 +17,20 @@ namespace emg {
 // SpMM launcher with an autotuned lane layout per (precision, K, row-length
 // class).  Tuning runs on the first large non-accumulating call it sees and
 // times every legal (V, NL) candidate with CUDA events.
+// One table serves the process: contexts of several threads look up and add
+// layouts under its lock; where two tune the same class, both use the first
+// one's choice.
 struct SpmmTuner {
   // (sizeof T, K, nonzeros-per-row class, row-count class) -> (V, NL)
-  std::map<std::tuple<int, int, int, int>, std::pair<int, int>> best;
-  bool allow_tuning = true;
-  int tuned_count = 0;
-  std::string report() const;
+  typedef std::tuple<int, int, int, int> Key;
+  typedef std::pair<int, int> Layout;
+  std::string report();
+  bool find(const Key &k, Layout &l);
+  Layout add(const Key &k, const Layout &l);
+
+ private:
+  std::mutex mu;
+  std::map<Key, Layout> best;
 };
 
 SpmmTuner &tuner();
