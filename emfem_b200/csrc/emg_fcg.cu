@@ -200,12 +200,13 @@ __global__ void __launch_bounds__(kThreads) fcg_dots_kernel(long pairs, int lhp,
 }
 
 // p = z - sum_j beta_j P_j over NJ directions from j0 on, beta_j = (z, S_j) /
-// eta_j of the active columns (slot[j]: ring slot of j; ieta = 1 / eta, for a
-// thread has only one pair)
+// eta_j of the active columns (slot[j]: ring slot of j).  A quotient and not
+// a product with a stored 1 / eta: eta below 2^-1024, of right-hand sides of
+// norm 1e-152, has no finite reciprocal
 template <bool SPLIT, int NJ>
 __global__ void __launch_bounds__(kThreads) fcg_direction_kernel(long pairs, int lhp, const double2 *z,
                                                                  Fcg::ZSplit zs, int j0, Dirs P, Slots slot,
-                                                                 const double2 *acc, const double2 *ieta,
+                                                                 const double2 *acc, const double2 *eta,
                                                                  const int2 *act, double2 *p) {
   pdl_trigger();
   const long i = blockIdx.x * (long)kThreads + threadIdx.x;
@@ -217,14 +218,14 @@ __global__ void __launch_bounds__(kThreads) fcg_direction_kernel(long pairs, int
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
     d[j] = acc[((j0 + j) << lhp) + c2];
-    e[j] = ieta[(slot.s[j0 + j] << lhp) + c2];
+    e[j] = eta[(slot.s[j0 + j] << lhp) + c2];
     pj[j] = reinterpret_cast<const double2 *>(P.p[j0 + j])[i];
   }
   double2 v = z_at<SPLIT>(i, lhp, z, zs);
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    v.x -= (on.x ? d[j].x * e[j].x : 0.0) * pj[j].x;
-    v.y -= (on.y ? d[j].y * e[j].y : 0.0) * pj[j].y;
+    v.x -= (on.x && e[j].x != 0.0 ? d[j].x / e[j].x : 0.0) * pj[j].x;
+    v.y -= (on.y && e[j].y != 0.0 ? d[j].y / e[j].y : 0.0) * pj[j].y;
   }
   p[i] = v;
 }
@@ -247,15 +248,15 @@ __global__ void __launch_bounds__(kThreads) fcg_step_kernel(long pairs, int lhp,
 }
 
 // x += alpha p, r -= alpha s (in every form), alpha = (p, r) / (p, s) of the
-// active columns from their sums.  The last block stores 1 / (p, s) and alpha, counts the iteration of every active column, retires the
-// converged ones (||r_c||^2 <= rtol^2 ||b_c||^2), flags NaN/Inf and clears the
-// sums (acc: the nacc of this iteration's passes, those of the step length at
-// kstep): status[0] = active columns left, status[1] = 1 + a non-finite column
-// (0: none)
+// active columns from their sums.  The last block stores (p, s) and alpha, counts
+// the iteration of every active column, retires the converged ones (||r_c||^2 <=
+// rtol^2 ||b_c||^2), flags NaN/Inf and clears the sums (acc: the nacc of this
+// iteration's passes, those of the step length at kstep): status[0] = active
+// columns left, status[1] = 1 + a non-finite column (0: none)
 __global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int lhp, const double2 *p,
                                                               const double2 *sv, double *const *xslot, double2 *r,
                                                               FcgFeed feed, double *acc, int kstep, int nacc,
-                                                              double *acc_rr, double *ieta, double *alpha, double *bn,
+                                                              double *acc_rr, double *eta, double *alpha, double *bn,
                                                               double rtol2, int *act, int *its, int *status,
                                                               unsigned *count) {
   pdl_trigger();
@@ -286,8 +287,8 @@ __global__ void __launch_bounds__(kThreads) fcg_update_kernel(long pairs, int lh
   __shared__ int left;
   if (threadIdx.x == 0) left = 0;
   if (threadIdx.x < hp) {  // blocks start on a row, so this thread's columns are c and c + 1
-    ieta[c] = ps0 != 0.0 ? 1.0 / ps0 : 0.0;
-    ieta[c + 1] = ps1 != 0.0 ? 1.0 / ps1 : 0.0;
+    eta[c] = ps0;
+    eta[c + 1] = ps1;
     alpha[c] = a0;
     alpha[c + 1] = a1;
   }
@@ -354,7 +355,7 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
     }
   }
   acc.alloc((size_t)(mmax + 4) * K);
-  ieta.alloc((size_t)mmax * K);
+  eta.alloc((size_t)mmax * K);
   alpha.alloc(K);
   bn.alloc(K);
   xslot.alloc(1);
@@ -389,7 +390,7 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
       add(P[j].p);
       add(S[j].p);
     }
-    for (const void *p : {(const void *)acc.p, (const void *)ieta.p, (const void *)alpha.p,
+    for (const void *p : {(const void *)acc.p, (const void *)eta.p, (const void *)alpha.p,
                           (const void *)bn.p, (const void *)xslot.p, (const void *)act.p, (const void *)itsd.p,
                           (const void *)status.p, (const void *)count.p, (const void *)feed.r32,
                           (const void *)feed.jf.y, (const void *)feed.jf.d, (const void *)feed.jd.y,
@@ -420,7 +421,7 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
     double *p = P[head].p, *sv = S[head].p;
     for (int j0 = 0; j0 == 0 || j0 < nprev; j0 += 4) {  // a later group goes on from p
       launch_chain(direction_of(zs && j0 == 0, std::min(4, nprev - j0)), dir_grid, kThreads, s, true, pairs, lhp,
-                   (const double2 *)(j0 ? p : z.p), z0, j0, Pd, sl, (const double2 *)acc.p, (const double2 *)ieta.p,
+                   (const double2 *)(j0 ? p : z.p), z0, j0, Pd, sl, (const double2 *)acc.p, (const double2 *)eta.p,
                    (const int2 *)act.p, (double2 *)p);
       EMG_LAUNCH_CHECK();
     }
@@ -430,7 +431,7 @@ int Fcg::solve(int n, int Kc, const std::function<void(const double *, double *)
     EMG_LAUNCH_CHECK();
     launch_chain(&fcg_update_kernel, pass_grid(pairs, 8), kThreads, s, true, pairs, lhp, (const double2 *)p,
                  (const double2 *)sv, xslot.p, (double2 *)r.p, feed, acc.p, kstep, kstep + 2 * K, acc_rr,
-                 ieta.p + (size_t)head * K, alpha.p, bn.p, rtol * rtol, act.p, itsd.p, status.p, count.p + 1);
+                 eta.p + (size_t)head * K, alpha.p, bn.p, rtol * rtol, act.p, itsd.p, status.p, count.p + 1);
     EMG_LAUNCH_CHECK();
   };
   auto run = [&](int head, int nprev) {

@@ -70,7 +70,7 @@ struct Fcg {
   DBuf<double> r, z;
   std::vector<DBuf<double>> P, S;  // previous directions and B-products (ring)
   DBuf<double> acc;                // sums in progress: mmax K (z, S_j), K (p, s), K (p, r), K (r, r), K (b, b)
-  DBuf<double> ieta, alpha, bn;  // ieta: 1 / (p, s) of the ring
+  DBuf<double> eta, alpha, bn;  // eta: (p, s) of the ring
   DBuf<double *> xslot;            // where the running solve's x lies (graphs outlive a solve)
   DBuf<int> act, itsd, status;     // per-column activity and iteration counts; active count, NaN flag
   DBuf<unsigned> count;            // blocks done per reducing kernel

@@ -140,3 +140,22 @@ def test_fcg_long_vectors(mmax):
         assert err.max() <= 1e-6, err
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("power", [-520, -515, -500, 0, 480])
+def test_pc_apply_scales(system, power):
+    """The preconditioner is linear: b scaled by a power of two gives x scaled
+    by it, also where the squares of its FCG are near the ends of the range (norms of b
+    from 1e-151 to 1e150; below, the squares of a solve to 1e-2 are subnormal
+    and lose its digits).  The order of the sums differs from run to run, by
+    1e-10 of x: the solve tests' 1e-6."""
+    c, colf, s, _ = system
+    c.process_options("-emg_amg_max_coarse 40")
+    c.assemble_matrix(0)
+    c.create_pc()
+    b = np.concatenate([s[:, 0].real, s[:, 0].imag])
+    b *= 2.0 ** -int(np.floor(np.log2(np.linalg.norm(b)))) * 2.0 ** 18
+    x0 = c.pc_apply_b(b)
+    x = c.pc_apply_b(b * 2.0 ** power)
+    x = x * 2.0 ** -(power // 2) * 2.0 ** -(power - power // 2)
+    assert np.linalg.norm(x - x0) <= 1e-6 * np.linalg.norm(x0)
