@@ -159,3 +159,24 @@ def test_pc_apply_scales(system, power):
     x = c.pc_apply_b(b * 2.0 ** power)
     x = x * 2.0 ** -(power // 2) * 2.0 ** -(power - power // 2)
     assert np.linalg.norm(x - x0) <= 1e-6 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("mmax", [1, 2, 3, 4, 5, 9])
+def test_fcg_groups_are_reached(system, fp32, mmax):
+    """test_fcg_truncations with inner solves long enough that the ring of directions
+    fills and wraps: more than mmax + 1 inner iterations per outer one."""
+    if fp32 and mmax > 4:
+        pytest.skip("refused with the FP32 preconditioner")
+    c, colf, s, exact = system
+    c.process_options(f"-emg_amg_max_coarse 40 -emg_block_fcg_mmax {mmax} -emg_block_inner_rtol 1e-6 "
+                      "-emg_block_inner_max_it 60")
+    try:
+        c.assemble_matrix(0)
+        x, infos = c.solve_block(colf[:4], s[:, :4], rtol=1e-8, max_it=200, inner_fp32=fp32)
+    finally:
+        c.process_options("-emg_block_fcg_mmax 2 -emg_block_inner_rtol 1e-2 -emg_block_inner_max_it 30")
+    assert all(i.reason == 0 for i in infos)
+    assert min(i.inner_its / i.outer_its for i in infos) > mmax + 1, [(i.inner_its, i.outer_its) for i in infos]
+    err = np.abs(x - exact[:, :4]).max(axis=0) / np.abs(exact[:, :4]).max(axis=0)
+    assert err.max() <= 1e-6, err
