@@ -478,9 +478,9 @@ __device__ __forceinline__ bool element_matrices(const ElemIn &in, int t, double
 // number as (f, e), and the operator the one that the nodal spaces and G^T B
 // are built from.  (In the air w sigma Ms is 1e-10 of C: rows that each
 // started from their own edge moved solutions by 4e-10.)
-// Bound: the data pipe of L1 (the gathers of a tet's data, each a pass per
-// lane, and the tile's read-modify-writes; C and Ms of a slot lie together for
-// those).  600k tets: 320 us scattered, 206 now; rows that differed from their
+// Bound: L1 at 68 % (the gathers of a tet's data, each a pass per lane, and the
+// tile's read-modify-writes; C and Ms of a slot lie together for those) and
+// latency, with 18 warps active per SM.  600k tets: 320 us scattered, 206 now; rows that differed from their
 // mirror took 193, 6 blocks per SM instead of 5 (8 bytes spilled) 205.
 constexpr int ASM_ROWS = 128;
 constexpr int ASM_SLOTS = ASM_ROWS * 18;  // a tile holds rows of 18 slots on average (36.9 KB)

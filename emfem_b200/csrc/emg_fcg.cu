@@ -12,8 +12,8 @@
 // sums.  With a last block in every reducing pass instead, 64-bit divisions
 // by the row width and 8 blocks per SM (dots / step length, us per pass):
 // 6.1k rows, 16 columns 5.9 / 4.8 -> 1.9 / 1.7, 100k rows, 8 columns 11.5 /
-// 8.5 -> 5.1 / 4.9, 150k rows, 32 columns 39 / 25 -> 14 / 17 (floor of the
-// last: 100 and 115 MB, 15 and 18 us; both partly from L2).  The direction
+// 8.5 -> 5.1 / 4.9, 150k rows, 32 columns 39 / 25 -> 14 / 17 (the last move 100
+// and 115 MB, 15 and 18 us if all of it came from HBM; part is in L2).  The direction
 // pays 1.8 us for its scalars at the smallest size.
 
 #include <cuda_runtime.h>

@@ -744,12 +744,13 @@ struct Omegas {
 
 // y = A(w_c) x or b - A(w_c) x: CL = K / V lanes of V columns per row, NL lanes
 // splitting its nonzeros, U nonzeros per lane and round; the index and value
-// loads of a round go out before its gathers.  The data pipe of L1 is the
-// busiest unit (66 % at K = 16, 1.81M rows; L2 21 %, DRAM 26 %): a warp-wide
-// load that touches several rows costs a pass per row, so few lanes per row
-// with two columns each share the three matrix loads of a nonzero best.
-// Measured: 806 -> 685 us at K = 16, 1.81M rows (V = 2, 3 blocks per SM; V = 1
-// 842, V = 4 789, two rows per warp with split nonzeros 1111).
+// loads of a round go out before its gathers.  L1 is the busiest unit
+// (64 % at K = 16, 357k rows, its data pipe 62 %; L2 20 %, DRAM 23 %): a
+// warp-wide load that touches several rows costs a pass per row, so few lanes per
+// row with two columns each share the three matrix loads of a nonzero best.
+// Measured at K = 16, 1.81M rows: whole calls 806 -> 699 us; the kernel 685 us
+// with V = 2 and 3 blocks per SM, 842 with V = 1, 789 with V = 4, 1111 with two
+// rows per warp and split nonzeros.
 template <int K, int V, int NL, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) spmm_complex_kernel(int n, const int *__restrict__ rp,
                                                            const int *__restrict__ ci, const double *__restrict__ Cv,
